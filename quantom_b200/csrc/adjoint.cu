@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(kAdjTB) k_adj_bonded(PhysDev d, const float4* 
                 const float4 o = make_float4((hvp ? a.dt * f.x.t : 0.f) - a.le * f.x.v,
                                              (hvp ? a.dt * f.y.t : 0.f) - a.le * f.y.v,
                                              (hvp ? a.dt * f.z.t : 0.f) - a.le * f.z.v, 0.f);
-                a.adj_term[slot0 + q] = o;
+                a.adj_term[d.bterm_pos[slot0 + q]] = o;
             }
             double2 acc = a.gterm[t];
             acc.x += (double)(a.dt * dg_dc * sg + a.le * dE_dc);
@@ -437,13 +437,16 @@ __global__ void __launch_bounds__(kAdjTB) k_adj_pair(PhysDev d, const float4* __
     if (i < d.n && g == 0) {
         float bx = 0.f, by = 0.f, bz = 0.f;
         const uint32_t oi = d.orig_of_sorted[i];
-        if (oi < (uint32_t)d.n_cp)
-            for (uint32_t q = d.bterm_off[oi]; q < d.bterm_off[oi + 1]; q++) {
-                const float4 tf = a.adj_term[d.bterm_slot[q]];
+        if (oi < (uint32_t)d.n_cp) {
+            const uint32_t q1 = d.bterm_off[oi + 1];
+#pragma unroll 4
+            for (uint32_t q = d.bterm_off[oi]; q < q1; q++) {
+                const float4 tf = a.adj_term[q];
                 bx += tf.x;
                 by += tf.y;
                 bz += tf.z;
             }
+        }
         float4 lx = a.lam_x[i];
         lx.x += a.dt * hx - a.le * fx + a.lr * rx + bx;
         lx.y += a.dt * hy - a.le * fy + a.lr * ry + by;

@@ -517,8 +517,8 @@ __device__ __forceinline__ void block_sums_fixed(double (&v)[K], double* out) {
 
 }  // namespace
 
-// One thread per bonded term: the forces on its atoms into its term_force
-// slots (w: each atom's share of the term's energy).  The step kernel that
+// One thread per bonded term: the forces on its atoms (w: each atom's share of
+// the term's energy), each into its atom's run of term_force (bterm_pos).  The step kernel that
 // follows is launched programmatically and starts right away; only the lanes
 // that gather these slots wait for this kernel.  ENERGY: per-block FP64 sums
 // of the bond, angle and dihedral energies and the virial into bpart.
@@ -557,8 +557,9 @@ __global__ void __launch_bounds__(kTB) k_bonded(PhysDev d, int cur) {
         }
         // w: each atom's share of the term's energy (per-particle potential energy)
         const float sh = ENERGY ? (float)(0.5 * eb) : 0.f;
-        d.term_force[2 * t + 0] = make_float4(-f * rx, -f * ry, -f * rz, sh);
-        d.term_force[2 * t + 1] = make_float4(f * rx, f * ry, f * rz, sh);
+        const uint32_t* at = d.bterm_pos + 2 * t;
+        d.term_force[at[0]] = make_float4(-f * rx, -f * ry, -f * rz, sh);
+        d.term_force[at[1]] = make_float4(f * rx, f * ry, f * rz, sh);
     } else if (t < d.n_bonds + d.n_angles) {
         const int a_ = t - d.n_bonds;
         const int4 ix = d.angle_idx[a_];
@@ -586,10 +587,10 @@ __global__ void __launch_bounds__(kTB) k_bonded(PhysDev d, int cur) {
             vir = (double)(ux * fix + uy * fiy + uz * fiz + vx * fkx + vy * fky + vz * fkz);
         }
         const float sh = ENERGY ? (float)(ea / 3.0) : 0.f;
-        const int base = 2 * d.n_bonds + 3 * a_;
-        d.term_force[base + 0] = make_float4(fix, fiy, fiz, sh);
-        d.term_force[base + 1] = make_float4(-fix - fkx, -fiy - fky, -fiz - fkz, sh);
-        d.term_force[base + 2] = make_float4(fkx, fky, fkz, sh);
+        const uint32_t* at = d.bterm_pos + 2 * d.n_bonds + 3 * a_;
+        d.term_force[at[0]] = make_float4(fix, fiy, fiz, sh);
+        d.term_force[at[1]] = make_float4(-fix - fkx, -fiy - fky, -fiz - fkz, sh);
+        d.term_force[at[2]] = make_float4(fkx, fky, fkz, sh);
     } else if (t < d.n_bonds + d.n_angles + d.n_dih) {
         const int q = t - d.n_bonds - d.n_angles;
         const int4 ix = d.dih_idx[q];
@@ -619,11 +620,11 @@ __global__ void __launch_bounds__(kTB) k_bonded(PhysDev d, int cur) {
         const float fkx = -flx + p * fix - r * flx, fky = -fly + p * fiy - r * fly, fkz = -flz + p * fiz - r * flz;
         if (ENERGY) ed = (double)par.y * (1.0 + (double)cv);
         const float sh = ENERGY ? (float)(0.25 * ed) : 0.f;
-        const int base = 2 * d.n_bonds + 3 * d.n_angles + 4 * q;
-        d.term_force[base + 0] = make_float4(fix, fiy, fiz, sh);
-        d.term_force[base + 1] = make_float4(fjx, fjy, fjz, sh);
-        d.term_force[base + 2] = make_float4(fkx, fky, fkz, sh);
-        d.term_force[base + 3] = make_float4(flx, fly, flz, sh);
+        const uint32_t* at = d.bterm_pos + 2 * d.n_bonds + 3 * d.n_angles + 4 * q;
+        d.term_force[at[0]] = make_float4(fix, fiy, fiz, sh);
+        d.term_force[at[1]] = make_float4(fjx, fjy, fjz, sh);
+        d.term_force[at[2]] = make_float4(fkx, fky, fkz, sh);
+        d.term_force[at[3]] = make_float4(flx, fly, flz, sh);
         if (ENERGY) {
             vir = (double)(b1x * fjx + b1y * fjy + b1z * fjz + (b1x + b2x) * fkx + (b1y + b2y) * fky +
                            (b1z + b2z) * fkz + (b1x + b2x + b3x) * flx + (b1y + b2y + b3y) * fly +
@@ -1011,8 +1012,10 @@ __device__ __forceinline__ void step_body(const PhysDev& d, int cur, int slot, c
             // kernel's list walk; wait for it only here)
             pdl_wait();
             float bx = 0.f, by = 0.f, bz = 0.f, bw = 0.f;
-            for (uint32_t q = d.bterm_off[oi]; q < d.bterm_off[oi + 1]; q++) {
-                const float4 tf = __ldcg(&d.term_force[d.bterm_slot[q]]);
+            const uint32_t q1 = d.bterm_off[oi + 1];
+#pragma unroll 4
+            for (uint32_t q = d.bterm_off[oi]; q < q1; q++) {
+                const float4 tf = __ldcg(&d.term_force[q]);
                 bx += tf.x;
                 by += tf.y;
                 bz += tf.z;

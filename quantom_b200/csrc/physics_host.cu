@@ -283,6 +283,9 @@ int phys_setup(const PhysHost& h, PhysDev& d, cudaStream_t s, std::vector<void*>
         boff[i + 1] = boff[i] + (uint32_t)slots[i].size();
         bslot.insert(bslot.end(), slots[i].begin(), slots[i].end());
     }
+    // where each term slot's force goes: its atom's run, at the slot's place in it
+    std::vector<uint32_t> bpos(d.n_term_slots);
+    for (size_t q = 0; q < bslot.size(); q++) bpos[bslot[q]] = (uint32_t)q;
 
     // cell grid (side >= rlist/2: the 5x5x5 neighbourhood covers rlist) and
     // Verlet-list capacity
@@ -311,7 +314,7 @@ int phys_setup(const PhysHost& h, PhysDev& d, cudaStream_t s, std::vector<void*>
         d.dih_idx = a.take<int4>(didx.size());
         d.dih_par = a.take<float4>(dpar.size());
         d.bterm_off = a.take<uint32_t>(boff.size());
-        d.bterm_slot = a.take<uint32_t>(bslot.size());
+        d.bterm_pos = a.take<uint32_t>(bpos.size());
     };
     size_t topo_bytes = 0;
     auto carve = [&](Arena& a) {
@@ -380,7 +383,7 @@ int phys_setup(const PhysHost& h, PhysDev& d, cudaStream_t s, std::vector<void*>
         put(d.dih_idx, didx.data(), sizeof(int4) * didx.size());
         put(d.dih_par, dpar.data(), sizeof(float4) * dpar.size());
         put(d.bterm_off, boff.data(), sizeof(uint32_t) * boff.size());
-        put(d.bterm_slot, bslot.data(), sizeof(uint32_t) * bslot.size());
+        put(d.bterm_pos, bpos.data(), sizeof(uint32_t) * bpos.size());
         cudaMemcpyAsync(d.cp_base, img.data(), topo_bytes, cudaMemcpyHostToDevice, s);   // pageable: copied at the call
     }
     cudaMemsetAsync(d.ccount, 0, sizeof(uint32_t) * d.n_cells, s);
