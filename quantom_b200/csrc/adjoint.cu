@@ -15,9 +15,11 @@
 // derivatives are reduced per block in FP64.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "adjoint.cuh"
 #include "physkern.cuh"
+#include "physmath.cuh"
 #include "refdev.cuh"
 
 namespace lima {
@@ -31,8 +33,54 @@ constexpr int kListEpoch = 10;
 
 __device__ __forceinline__ float mimg_a(float d, float L, float invL) { return d - L * rintf(d * invL); }
 
-__device__ __forceinline__ uint32_t nl_at(const PhysDev& d, int i, int k) {
-    return nl_word((uint32_t)d.n_pad, (uint32_t)i, (uint32_t)k);
+// Minimum image of a difference of two coordinates in [0, L): the rounding of
+// d / L (|d / L| < 1) by adding and subtracting 1.5 * 2^23, three operations of
+// the FP32 pipes (rintf takes a slower one).
+__device__ __forceinline__ float mimg_add(float d, float L, float invL) {
+    const float k = fmaf(d, invL, 12582912.f) - 12582912.f;
+    return fmaf(-L, k, d);
+}
+
+// 1 / x to about half an ulp: the special-function unit's reciprocal and one
+// Newton step (x positive, far from the denormal and overflow ranges)
+__device__ __forceinline__ float rcp_newton(float x) {
+    const float r = rcp_approx(x);
+    return fmaf(r, fmaf(-x, r, 1.f), r);
+}
+
+// f(slot j, position) for one lane's entries of particle i's list, of the LANES
+// lanes that share it: lane 8 h + g takes column g of the chunks h, h + LANES /
+// 8, ... (nl_word), four entries per vector load and four gathers in flight.
+template <int LANES, typename ID, typename F>
+__device__ __forceinline__ void for_entries(const PhysDev& d, const float4* __restrict__ pos, int i, int lane, int cnt,
+                                            F f) {
+    using V = typename std::conditional<sizeof(ID) == 2, uint2, uint4>::type;
+    constexpr int H = LANES / kGroup;
+    const int g = lane % kGroup, h = lane / kGroup;
+    const size_t cstride = (size_t)d.n_pad * kGroup;
+    const V* __restrict__ col = reinterpret_cast<const V*>(d.nl) + (size_t)i * kGroup + g + h * cstride;
+    for (int k = h * kListChunk + g; k < cnt; k += H * kListChunk, col += H * cstride) {
+        const V v = __ldg(col);
+        uint32_t j[4];
+        if constexpr (sizeof(ID) == 2) {
+            j[0] = v.x & 0xffffu;
+            j[1] = v.x >> 16;
+            j[2] = v.y & 0xffffu;
+            j[3] = v.y >> 16;
+        } else {
+            j[0] = v.x;
+            j[1] = v.y;
+            j[2] = v.z;
+            j[3] = v.w;
+        }
+        const int m = min(4, (cnt - k + kGroup - 1) / kGroup);   // words past the count are not ids
+        float4 p[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) p[u] = __ldg(pos + (u < m ? j[u] : j[0]));
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (u < m) f(j[u], p[u]);
+    }
 }
 
 __device__ __forceinline__ double warp_sum_d(double v) {
@@ -60,13 +108,13 @@ __device__ __forceinline__ void bspline3(float r, float inv_dr, int& k0, float w
 struct LJ1 {
     float ph, f, fp, dph_ds, df_ds;
 };
-__device__ __forceinline__ LJ1 lj1(const PhysDev& d, float r2, float sig2) {
-    const float u = 1.f / r2;
+// isig = 1 / sigma.
+__device__ __forceinline__ LJ1 lj1(const PhysDev& d, float r2, float sig2, float isig) {
+    const float u = rcp_newton(r2);
     const float s2 = sig2 * u, s6 = s2 * s2 * s2, s12 = s6 * s6;
     const float ph = s12 - s6;
     const float f = 6.f * u * (2.f * s12 - s6);
     const float fp = -6.f * u * u * (14.f * s12 - 4.f * s6);
-    const float isig = rsqrtf(sig2);
     const float dph_ds = (12.f * s12 - 6.f * s6) * isig;
     const float df_ds = 6.f * u * (24.f * s12 - 6.f * s6) * isig;
     // C2 switch S(t), t = (rc^2 - r^2) / (rc^2 - r_on^2)
@@ -101,59 +149,67 @@ struct AdjArgs {
 };
 
 // --------------------------------------------------------------- loss pass --
-// The block's occupancies accumulate in shared memory as 64-bit fixed point
-// in units of 2^-32 (each half weight, at most 0.375, converted from FP32;
-// integer sums do not depend on their order, so the block's sums are
-// deterministic), then go to FP64 once per bin and block.
-constexpr double kHistUnit = 1.0 / 4294967296.0;   // 2^-32
-
-__global__ void __launch_bounds__(kAdjTB) k_loss_pairs(PhysDev d, const float4* __restrict__ pos, int n_bins,
-                                                       float inv_dr, float supp2, double inv_n,
-                                                       double* __restrict__ U_out, double* __restrict__ h_out) {
-    __shared__ unsigned long long s_hist[LIMA_LOSS_MAX_BINS];
-    __shared__ double s_e[kAdjTB / 32];
+// A lane keeps occupancies of its own, one column of a [bins + 4][32] array per
+// warp in shared memory (a row past either end takes the weights that fall
+// outside, so no bin is tested): each of a pair's three weights is a plain load,
+// add and store with no bank conflict and no atomic.  A lane adds a few FP32
+// weights per bin; the block's lanes are summed in FP64.  8,192 particles, 50
+// bins on one B200: shared-memory 64-bit atomics, three per pair, took 87 us.
+constexpr int kLossTB = 128;
+template <typename ID>
+__global__ void __launch_bounds__(kLossTB) k_loss_pairs(PhysDev d, const float4* __restrict__ pos, int n_bins,
+                                                        float inv_dr, float supp2, double inv_n,
+                                                        double* __restrict__ U_out, double* __restrict__ h_out) {
+    extern __shared__ float s_hist[];   // [warps][n_bins + 4][32]
+    __shared__ double s_e[kLossTB / 32];
     __shared__ float2 s_tab[kMaxTypes * kMaxTypes];
-    const int nt2 = d.n_types * d.n_types;
+    const int nt2 = d.n_types * d.n_types, rows = n_bins + 4;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (int q = threadIdx.x; q < nt2; q += blockDim.x) s_tab[q] = d.lj_table[q];
-    for (int b = threadIdx.x; b < n_bins; b += blockDim.x) s_hist[b] = 0ull;
+    float* mine = s_hist + (size_t)w * rows * 32 + lane;   // the lane's column
+    for (int b = 0; b < rows; b++) mine[b * 32] = 0.f;
     __syncthreads();
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) / kGroup;
     const int g = threadIdx.x % kGroup;
     float e = 0.f;
     if (i < d.n) {
         const float4 pi = pos[i];
-        const int ti = __float_as_int(pi.w);
+        const float2* row = s_tab + __float_as_int(pi.w) * d.n_types;
         const int cnt = (int)d.nl_cnt[i];
-        for (int k = g; k < cnt; k += kGroup) {
-            const uint32_t j = nl_load(d, nl_at(d, i, k));
-            const float4 pj = pos[j];
-            const float dx = mimg_a(pi.x - pj.x, d.L, d.invL), dy = mimg_a(pi.y - pj.y, d.L, d.invL),
-                        dz = mimg_a(pi.z - pj.z, d.L, d.invL);
+        for_entries<kGroup, ID>(d, pos, i, g, cnt, [&](uint32_t, float4 pj) {
+            const float dx = mimg_add(pi.x - pj.x, d.L, d.invL), dy = mimg_add(pi.y - pj.y, d.L, d.invL),
+                        dz = mimg_add(pi.z - pj.z, d.L, d.invL);
             const float r2 = dx * dx + dy * dy + dz * dz;
-            if (r2 < d.rc2) {
-                const float2 tab = s_tab[ti * d.n_types + __float_as_int(pj.w)];
-                e += 0.5f * tab.y * lj1(d, r2, tab.x).ph;
-            }
+            const float2 tab = row[__float_as_int(pj.w)];
+            const float s2 = tab.x * rcp_newton(r2), s6 = s2 * s2 * s2;
+            const float t = __saturatef((d.rc2 - r2) * d.inv_sw_d);   // 0 beyond r_c
+            e += tab.y * fmaf(s6, s6, -s6) * (t * t * t * fmaf(t, fmaf(6.f, t, -15.f), 10.f));
             if (r2 < supp2) {
                 int k0;
-                float w[3], dw[3];
-                bspline3(sqrtf(r2), inv_dr, k0, w, dw);
-#pragma unroll
-                for (int q = 0; q < 3; q++)
-                    if (k0 + q >= 0 && k0 + q < n_bins)   // each pair is seen from both ends: half weight
-                        atomicAdd(&s_hist[k0 + q], (unsigned long long)__float2ull_rn(0.5f * w[q] * 4294967296.f));
+                float wt[3], dw[3];
+                bspline3(sqrtf(r2), inv_dr, k0, wt, dw);
+                float* q = mine + (k0 + 1) * 32;   // k0 is -1 .. n_bins
+                q[0] += wt[0];
+                q[32] += wt[1];
+                q[64] += wt[2];
             }
-        }
+        });
     }
     // energy: FP64 warp sums, then the block's warps in a fixed order
-    const double ew = warp_sum_d((double)e);
-    if ((threadIdx.x & 31) == 0) s_e[threadIdx.x >> 5] = ew;
+    const double ew = warp_sum_d(0.5 * (double)e);
+    if (lane == 0) s_e[w] = ew;
     __syncthreads();
-    for (int b = threadIdx.x; b < n_bins; b += blockDim.x)
-        if (s_hist[b]) atomicAdd(&h_out[b], (double)s_hist[b] * kHistUnit * inv_n);
+    // each pair is seen from both ends: half weight
+    for (int b = w; b < n_bins; b += kLossTB / 32) {
+        double v = 0.0;
+#pragma unroll
+        for (int q = 0; q < kLossTB / 32; q++) v += (double)s_hist[((size_t)q * rows + b + 1) * 32 + lane];
+        v = warp_sum_d(v);
+        if (lane == 0 && v != 0.0) atomicAdd(&h_out[b], 0.5 * v * inv_n);
+    }
     if (threadIdx.x == 0) {
         double v = 0.0;
-        for (int q = 0; q < kAdjTB / 32; q++) v += s_e[q];
+        for (int q = 0; q < kLossTB / 32; q++) v += s_e[q];
         if (v != 0.0) atomicAdd(U_out, v);
     }
 }
@@ -336,52 +392,68 @@ __global__ void k_adj_prep(PhysDev d, AdjArgs a, float4* __restrict__ lam_v, flo
     wv[i] = make_float4(mx * im, my * im, mz * im, 0.f);
 }
 
-template <bool HVP, bool LOSS>
-__global__ void __launch_bounds__(kAdjTB) k_adj_pair(PhysDev d, const float4* __restrict__ pos, AdjArgs a,
-                                                     const double* __restrict__ hist_n,
-                                                     const double* __restrict__ target) {
-    __shared__ float2 s_tab[kMaxTypes * kMaxTypes];
-    __shared__ float s_c[LIMA_LOSS_MAX_BINS];
-    __shared__ float s_par[2 * kMaxTypes];
-    __shared__ double s_g[2 * kMaxTypes];
+// kGroup lanes per particle (pair_lanes).  Every entry is evaluated (beyond r_c the switch and
+// its derivatives are zero, beyond the last bin the staged occupancy error is),
+// so a warp's lanes stay together.  The quotients of the per-type chain rule
+// (sigma_ij = (s_a + s_b) / 2, eps_ij = sqrt(e_a e_b)) are a table per type
+// pair.  The derivatives that land on the neighbour's type go to a column of
+// the lane's own in shared memory ([2 types][32] per warp: no conflicts, no
+// atomics; one type: registers), and are summed over the block in FP64.
+// 8,192 particles on one B200: 55 us with per-thread arrays indexed by type
+// (local memory) and four IEEE divisions an entry.
+constexpr int kAdjPairTB = 128;
+template <bool HVP, bool LOSS, typename ID, int LANES>
+__global__ void __launch_bounds__(kAdjPairTB) k_adj_pair(PhysDev d, const float4* __restrict__ pos, AdjArgs a,
+                                                         const double* __restrict__ hist_n,
+                                                         const double* __restrict__ target) {
+    extern __shared__ float4 s_dyn[];
+    // per type pair: (sigma^2, 4 eps, 1 / sigma, 0) and d eps_ij / d eps of i's and j's type
+    __shared__ float s_c[LIMA_LOSS_MAX_BINS + 8];   // occupancy error of bin b at b + 1, zero outside
     const int nt = a.n_types;
-    for (int q = threadIdx.x; q < nt * nt; q += blockDim.x) s_tab[q] = d.lj_table[q];
-    for (int q = threadIdx.x; q < 2 * nt; q += blockDim.x) {
-        s_par[q] = a.par[q];
-        s_g[q] = 0.0;
+    float4* s_tab = s_dyn;
+    float2* s_de = reinterpret_cast<float2*>(s_dyn + nt * nt);
+    float* s_g = reinterpret_cast<float*>(s_de + nt * nt + (nt * nt & 1));   // [warps][2 nt][32]
+    for (int q = threadIdx.x; q < nt * nt; q += blockDim.x) {
+        const float2 t = d.lj_table[q];
+        s_tab[q] = make_float4(t.x, t.y, rsqrtf(t.x), 0.f);
+        const float ei = a.par[nt + q / nt], ej = a.par[nt + q % nt], e = 0.25f * t.y;
+        s_de[q] = make_float2(ei > 0.f ? e / (2.f * ei) : 0.f, ej > 0.f ? e / (2.f * ej) : 0.f);
     }
     if (LOSS)
-        for (int q = threadIdx.x; q < a.n_bins; q += blockDim.x) s_c[q] = (float)(hist_n[q] - target[q]);
+        for (int q = threadIdx.x; q < LIMA_LOSS_MAX_BINS + 8; q += blockDim.x)
+            s_c[q] = q >= 1 && q <= a.n_bins ? (float)(hist_n[q - 1] - target[q - 1]) : 0.f;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const bool one = nt == 1;
+    float* mine = s_g + (size_t)w * 2 * nt * 32 + lane;   // the lane's column
+    for (int q = 0; q < 2 * nt; q++) mine[q * 32] = 0.f;
     __syncthreads();
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / kGroup;
-    const int g = threadIdx.x % kGroup;
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / LANES;
+    const int g = threadIdx.x % LANES;
     float hx = 0.f, hy = 0.f, hz = 0.f;   // dt * sum J (w_i - w_j)  (dt applied at the end)
     float fx = 0.f, fy = 0.f, fz = 0.f;   // LJ force on i
     float rx = 0.f, ry = 0.f, rz = 0.f;   // sum G(r) d
     float gs_a = 0.f, ge_a = 0.f;         // parameter derivatives landing on i's type
-    float gs_b[kMaxTypes], ge_b[kMaxTypes];
-    for (int q = 0; q < nt; q++) gs_b[q] = ge_b[q] = 0.f;
+    float gs_1 = 0.f, ge_1 = 0.f;         // on j's type, where there is one type
     int ti = 0;
     if (i < d.n) {
         const float4 pi = pos[i];
         ti = __float_as_int(pi.w);
         const float4 wi = HVP ? a.wv[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float eps_a = s_par[nt + ti];
         const int cnt = (int)d.nl_cnt[i];
-        for (int k = g; k < cnt; k += kGroup) {
-            const uint32_t j = nl_load(d, nl_at(d, i, k));
-            const float4 pj = pos[j];
-            const float dx = mimg_a(pi.x - pj.x, d.L, d.invL), dy = mimg_a(pi.y - pj.y, d.L, d.invL),
-                        dz = mimg_a(pi.z - pj.z, d.L, d.invL);
+        const bool rdf = LOSS && a.lr != 0.f;
+        const float hdt = 0.5f * a.dt, hle = 0.5f * a.le;
+        const int kmax = a.n_bins + 1;
+        for_entries<LANES, ID>(d, pos, i, g, cnt, [&](uint32_t j, float4 pj) {
+            const float dx = mimg_add(pi.x - pj.x, d.L, d.invL), dy = mimg_add(pi.y - pj.y, d.L, d.invL),
+                        dz = mimg_add(pi.z - pj.z, d.L, d.invL);
             const float r2 = dx * dx + dy * dy + dz * dz;
-            if (r2 >= d.rc2) continue;
-            const int tj = __float_as_int(pj.w);
-            const float2 tab = s_tab[ti * nt + tj];
+            const int tj = __float_as_int(pj.w), tt = ti * nt + tj;
+            const float4 tab = s_tab[tt];
             const float e4 = tab.y;   // 4 eps_ij
-            const LJ1 l = lj1(d, r2, tab.x);
+            const LJ1 l = lj1(d, r2, tab.x, tab.z);
             float dsig = 0.f, deps4 = 0.f;   // d/d sigma_ij and d/d (4 eps_ij) of this visit
             if (HVP) {
-                const float4 wj = a.wv[j];
+                const float4 wj = __ldg(a.wv + j);
                 const float ux = wi.x - wj.x, uy = wi.y - wj.y, uz = wi.z - wj.z;
                 const float du = dx * ux + dy * uy + dz * uz;
                 const float c1 = e4 * l.f, c2 = 2.f * e4 * l.fp * du;
@@ -389,41 +461,47 @@ __global__ void __launch_bounds__(kAdjTB) k_adj_pair(PhysDev d, const float4* __
                 hy += c1 * uy + c2 * dy;
                 hz += c1 * uz + c2 * dz;
                 // half of dt (w_i - w_j) . dF_i/dtheta (the other half comes from j's visit)
-                dsig += 0.5f * a.dt * du * e4 * l.df_ds;
-                deps4 += 0.5f * a.dt * du * l.f;
+                dsig += hdt * du * e4 * l.df_ds;
+                deps4 += hdt * du * l.f;
             }
             if (LOSS) {
-                fx += e4 * l.f * dx;
-                fy += e4 * l.f * dy;
-                fz += e4 * l.f * dz;
-                dsig += 0.5f * a.le * e4 * l.dph_ds;
-                deps4 += 0.5f * a.le * l.ph;
-                if (a.lr != 0.f && r2 < a.supp2) {
+                const float f = e4 * l.f;
+                fx += f * dx;
+                fy += f * dy;
+                fz += f * dz;
+                dsig += hle * e4 * l.dph_ds;
+                deps4 += hle * l.ph;
+                if (rdf) {
                     const float r = sqrtf(r2);
                     int k0;
-                    float w[3], dw[3];
-                    bspline3(r, a.inv_dr, k0, w, dw);
-                    float G = 0.f;
-#pragma unroll
-                    for (int q = 0; q < 3; q++)
-                        if (k0 + q >= 0 && k0 + q < a.n_bins) G += s_c[k0 + q] * dw[q];
-                    G /= r;
+                    float wt[3], dw[3];
+                    bspline3(r, a.inv_dr, k0, wt, dw);
+                    k0 = min(k0, kmax);   // past the support: zeros
+                    const float* c = s_c + k0 + 1;
+                    const float G = (c[0] * dw[0] + c[1] * dw[1] + c[2] * dw[2]) * rcp_newton(r);
                     rx += G * dx;
                     ry += G * dy;
                     rz += G * dz;
                 }
             }
-            // chain to the per-type parameters: sigma_ij = (s_a + s_b)/2, eps_ij = sqrt(e_a e_b)
-            const float eps_ab = 0.25f * e4, eps_b = s_par[nt + tj];
-            const float de = 4.f * deps4;   // d/d eps_ij
-            gs_a += 0.5f * dsig;
-            gs_b[tj] += 0.5f * dsig;
-            if (eps_a > 0.f) ge_a += de * eps_ab / (2.f * eps_a);
-            if (eps_b > 0.f) ge_b[tj] += de * eps_ab / (2.f * eps_b);
-        }
+            // chain to the per-type parameters
+            const float2 de = s_de[tt];
+            const float hs = 0.5f * dsig, d4 = 4.f * deps4;   // d/d eps_ij
+            gs_a += hs;
+            ge_a += d4 * de.x;
+            if (one) {
+                gs_1 += hs;
+                ge_1 += d4 * de.y;
+            } else {
+                mine[tj * 32] += hs;
+                mine[(nt + tj) * 32] += d4 * de.y;
+            }
+        });
+        mine[ti * 32] += gs_a + gs_1;   // one type: gs_1 is its other half
+        mine[(nt + ti) * 32] += ge_a + ge_1;
     }
 #pragma unroll
-    for (int o = kGroup / 2; o > 0; o >>= 1) {
+    for (int o = LANES / 2; o > 0; o >>= 1) {
         hx += __shfl_xor_sync(0xffffffffu, hx, o);
         hy += __shfl_xor_sync(0xffffffffu, hy, o);
         hz += __shfl_xor_sync(0xffffffffu, hz, o);
@@ -453,23 +531,15 @@ __global__ void __launch_bounds__(kAdjTB) k_adj_pair(PhysDev d, const float4* __
         lx.z += a.dt * hz - a.le * fz + a.lr * rz + bz;
         a.lam_x[i] = lx;
     }
-    // parameter derivatives: lane -> per-type slots -> block (FP64) -> global
-    const int lane = threadIdx.x & 31;
-    for (int q = 0; q < nt; q++) {
-        float s = gs_b[q] + (q == ti ? gs_a : 0.f);
-        float e = ge_b[q] + (q == ti ? ge_a : 0.f);
-        for (int o = 16; o > 0; o >>= 1) {
-            s += __shfl_down_sync(0xffffffffu, s, o);
-            e += __shfl_down_sync(0xffffffffu, e, o);
-        }
-        if (lane == 0) {
-            if (s != 0.f) atomicAdd(&s_g[q], (double)s);
-            if (e != 0.f) atomicAdd(&s_g[nt + q], (double)e);
-        }
-    }
     __syncthreads();
-    for (int q = threadIdx.x; q < 2 * nt; q += blockDim.x)
-        if (s_g[q] != 0.0) atomicAdd(&a.gtheta[q], s_g[q]);
+    // parameter derivatives: the block's lanes in FP64, then global
+    for (int q = w; q < 2 * nt; q += kAdjPairTB / 32) {
+        double v = 0.0;
+#pragma unroll
+        for (int k = 0; k < kAdjPairTB / 32; k++) v += (double)s_g[((size_t)k * 2 * nt + q) * 32 + lane];
+        v = warp_sum_d(v);
+        if (lane == 0 && v != 0.0) atomicAdd(&a.gtheta[q], v);
+    }
 }
 
 // ---------------------------------------------------------- state moves ---
@@ -694,6 +764,15 @@ int phys_params_set(PhysDev& d, PhysParams& pp, const double* theta, std::string
 // ------------------------------------------------------------------ passes --
 namespace {
 
+// Lanes that share one particle's list in the adjoint pair kernel: 8, and 16
+// in boxes whose 8-lane grid leaves most of an SM's warps unfilled.  A 50-step
+// gradient of 1,948 particles took 6.44 ms with 8, 5.82 with 16, 5.88 with 32;
+// 40 steps of 5,040 particles 5.54, 5.25, 5.82; 200 steps of 8,192 particles
+// 26.3, 27.6, 30.8 (with the loss kernel on as many lanes).  The loss kernel
+// keeps 8: more lanes are more columns of occupancies to clear and sum (200
+// steps of 8,192 particles: 11.5 ms with 8, 14.1 with 16).
+int pair_lanes(int n) { return n < 6144 ? 16 : kGroup; }
+
 struct Runner {
     PhysDev d;           // copy with fixed-period list semantics (stale -> error)
     AdjBuffers& A;
@@ -702,7 +781,7 @@ struct Runner {
     float inv_dr, supp2;
     int tb = 256;
     int blocks_n() const { return (d.n + tb - 1) / tb; }
-    int blocks_pair() const { return (int)(((size_t)d.n_pad * kGroup + kAdjTB - 1) / kAdjTB); }
+    int blocks_pair(int threads, int lanes) const { return (int)(((size_t)d.n * lanes + threads - 1) / threads); }
     int blocks_terms() const { return std::max(1, (d.n_bonds + d.n_angles + d.n_dih + kAdjTB - 1) / kAdjTB); }
 
     void save(int cur, int k) { k_save<<<blocks_n(), tb, 0, s>>>(d, cur, A.ck_x + (size_t)k * d.n, A.ck_v + (size_t)k * d.n); }
@@ -712,11 +791,40 @@ struct Runner {
     }
     // energy and occupancies of the state in parity cur -> U[n], hist[n]
     void loss_pass(int cur, const float4* pos, const float4* po, int n) {
-        k_loss_pairs<<<blocks_pair(), kAdjTB, 0, s>>>(d, pos, n_bins, inv_dr, supp2, 1.0 / d.n, A.U + n,
-                                                     A.hist + (size_t)n * n_bins);
-        AdjArgs a{};
-        k_adj_bonded<0><<<blocks_terms(), kAdjTB, 0, s>>>(d, po, a, 0, A.U + n);
+        const size_t smem = sizeof(float) * 32 * (kLossTB / 32) * (n_bins + 4);
+        auto run = [&](auto kernel) {
+            if (smem > 40 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            kernel<<<blocks_pair(kLossTB, kGroup), kLossTB, smem, s>>>(d, pos, n_bins, inv_dr, supp2, 1.0 / d.n, A.U + n,
+                                                               A.hist + (size_t)n * n_bins);
+        };
+        if (d.nl16) run(k_loss_pairs<uint16_t>);
+        else run(k_loss_pairs<uint32_t>);
+        if (d.n_bonds + d.n_angles + d.n_dih > 0) {
+            AdjArgs a{};
+            k_adj_bonded<0><<<blocks_terms(), kAdjTB, 0, s>>>(d, po, a, 0, A.U + n);
+        }
         (void)cur;
+    }
+    // one adjoint pair pass over the state xs (hist_n: its occupancies, with a loss term)
+    template <bool HVP, bool LOSS>
+    void adj_pair(const float4* xs, const AdjArgs& a, const double* hist_n) {
+        const int nt2 = a.n_types * a.n_types;
+        const size_t smem = sizeof(float4) * nt2 + sizeof(float2) * (nt2 + (nt2 & 1)) +
+                            sizeof(float) * 32 * (kAdjPairTB / 32) * 2 * a.n_types;
+        auto run = [&](auto kernel) {
+            if (smem > 40 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            kernel<<<blocks_pair(kAdjPairTB, pair_lanes(d.n)), kAdjPairTB, smem, s>>>(d, xs, a, hist_n, A.target);
+        };
+        if (pair_lanes(d.n) == 16) {
+            if (d.nl16) run(k_adj_pair<HVP, LOSS, uint16_t, 16>);
+            else run(k_adj_pair<HVP, LOSS, uint32_t, 16>);
+        } else {
+            if (d.nl16) run(k_adj_pair<HVP, LOSS, uint16_t, kGroup>);
+            else run(k_adj_pair<HVP, LOSS, uint32_t, kGroup>);
+        }
+    }
+    void adj_bonded(const float4* xo, const AdjArgs& a, int hvp) {
+        if (d.n_bonds + d.n_angles + d.n_dih > 0) k_adj_bonded<1><<<blocks_terms(), kAdjTB, 0, s>>>(d, xo, a, hvp, nullptr);
     }
 };
 
@@ -858,7 +966,6 @@ int adj_run(const PhysDev& d0, int cur, const PhysParams& pp, AdjBuffers& A, std
         a.par = A.par;
         a.gtheta = A.gtheta;
         a.gterm = A.gterm;
-        const int pb = R.blocks_pair(), tbk = R.blocks_terms();
         for (int k = K - 1; k >= 0; k--) {
             const int n0 = k * C, len = std::min(C, T - n0);
             R.restore(cur, k);
@@ -885,8 +992,8 @@ int adj_run(const PhysDev& d0, int cur, const PhysParams& pp, AdjBuffers& A, std
                 a.lr = lr;
                 const float4* xs = A.seg_x + (size_t)q * d.n_pad;
                 const float4* xo = A.seg_xo + (size_t)q * std::max(d.n_cp, 1);
-                k_adj_bonded<1><<<tbk, kAdjTB, 0, s>>>(d, xo, a, 0, nullptr);
-                k_adj_pair<false, true><<<pb, kAdjTB, 0, s>>>(d, xs, a, A.hist + (size_t)(n0 + q) * nb, A.target);
+                R.adj_bonded(xo, a, 0);
+                R.adj_pair<false, true>(xs, a, A.hist + (size_t)(n0 + q) * nb);
             }
             int epoch = (len - 1) / kListEpoch;   // the list built last
             for (int q = len - 1; q >= 0; q--) {
@@ -900,11 +1007,11 @@ int adj_run(const PhysDev& d0, int cur, const PhysParams& pp, AdjBuffers& A, std
                 const float4* xs = A.seg_x + (size_t)q * d.n_pad;
                 const float4* xo = A.seg_xo + (size_t)q * std::max(d.n_cp, 1);
                 k_adj_prep<<<R.blocks_n(), R.tb, 0, s>>>(d, a, A.lam_v, A.wv);
-                k_adj_bonded<1><<<tbk, kAdjTB, 0, s>>>(d, xo, a, 1, nullptr);
+                R.adj_bonded(xo, a, 1);
                 if (has_loss)
-                    k_adj_pair<true, true><<<pb, kAdjTB, 0, s>>>(d, xs, a, A.hist + (size_t)(n0 + q) * nb, A.target);
+                    R.adj_pair<true, true>(xs, a, A.hist + (size_t)(n0 + q) * nb);
                 else
-                    k_adj_pair<true, false><<<pb, kAdjTB, 0, s>>>(d, xs, a, nullptr, A.target);
+                    R.adj_pair<true, false>(xs, a, nullptr);
             }
             k_to_orig<<<R.blocks_n(), R.tb, 0, s>>>(d, A.lam_x, A.lam_xo);
             k_to_orig<<<R.blocks_n(), R.tb, 0, s>>>(d, A.lam_v, A.lam_vo);
