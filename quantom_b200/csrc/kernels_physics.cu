@@ -64,12 +64,6 @@ __device__ __forceinline__ void cell_xyz(const PhysDev& d, float4 p, int& cx, in
     cz = min(max((int)(p.z * inv), 0), d.m - 1);
 }
 
-__device__ __forceinline__ bool excluded(const PhysDev& d, uint32_t oi, uint32_t oj) {
-    for (uint32_t q = d.excl_off[oi]; q < d.excl_off[oi + 1]; q++)
-        if (d.excl_ids[q] == oj) return true;
-    return false;
-}
-
 }  // namespace
 
 // ----------------------------------------------------- counting sort by cell ---
@@ -185,22 +179,32 @@ __global__ void k_set_xref(PhysDev d, const float4* __restrict__ pos) {
 }
 
 
-// Verlet-list build: one warp per 8 consecutive particles of the cell order,
-// 4 lanes per particle (lane = 4 p + s).  The warp's particles are taken in
-// groups that share a home column (cells (x, y, *)) and a z-window of at most
-// m-4 cells; lanes outside the current group idle.  For a group, each of the
-// 25 columns around it is culled when the xy gap between the group's bounding
+// Verlet-list build: one warp per P consecutive particles of the cell order.
+// The warp's particles are taken in groups that share a home column (cells
+// (x, y, *)) and a z-window of at most m-4 cells.  For a group, each of the 25
+// columns around it is culled when the xy gap between the group's bounding
 // box and the column exceeds r_list, and otherwise contributes the cells that
 // the group's z-range, widened by the reach sqrt(r_list^2 - gap^2), overlaps:
 // one or two contiguous slot ranges of the cell order (at most m cells).  The
-// ranges are walked as one stream of candidates, 32 at a time: each lane
-// fetches one (the next batch while the current one is tested), shifts it
-// into the home frame by whole box lengths and stages it in shared memory.
-// Slice s of a particle tests candidates s, s+4, ..., drops itself and
-// bonded exclusions, and the slices' hit masks are merged with xor-shuffles;
-// each lane then writes its hits at their rank in the merged mask, so rows
-// list their neighbours in candidate order (deterministic).  Boxes with fewer
-// than 5 cells per side stream all particles with the minimum image.
+// ranges are walked as one stream of candidates, lane = candidate, 32 at a
+// time (the next 32 in flight while these are tested), shifted into the home
+// frame by whole box lengths.  Each particle's hits among them are a ballot:
+// the hit of rank r is appended to the particle's row in shared memory, r
+// entries past its count, by a predicated store.  At the end bonded exclusions
+// are taken out of the rows of the particles that have any, and the rows go to
+// the list in whole chunk columns, one vector store per lane.  Rows list their
+// neighbours in stream order (deterministic).  Boxes with fewer than 5 cells
+// per side stream all particles with the minimum image.
+//
+// Bound: issue slots (the candidate's range and address, the hits' ranks), and
+// latency where there are few warps; the list is written once.  So the hits
+// are ranked by ballots with predicated stores (8 particles a warp, 4 lanes a
+// particle walking the candidates took ~50 instructions per 32 tests for hit
+// masks, ranks and branches), loops run on values the compiler knows to be
+// uniform, exclusions cost only the rows that have any, and small boxes put
+// one particle on a warp (kBuildOneBelow).  A host-issued rebuild, sort and
+// launches included, on one B200 (before -> now): 4,096 particles 110 -> 47
+// us, 8,192 120 -> 61, 32,024 153 -> 110, 258,192 683 -> 557.
 // pos/orig: positions and orig ids by slot.  items (nullable): the cell order
 // as a list of slots when the particles were not moved into it (in-place
 // rebuild).  copy_cur >= 0: the particles were permuted into the tmp arrays
@@ -208,102 +212,206 @@ __global__ void k_set_xref(PhysDev d, const float4* __restrict__ pos) {
 // into the step arrays of parity copy_cur (the rebuild's last copy).
 namespace {
 
-constexpr int kBuildSlices = 4;                  // lanes per particle
-constexpr int kBuildPerWarp = 32 / kBuildSlices; // particles per warp
-constexpr int kMaxRanges = 50;                   // 25 columns, one or two slot ranges each
+constexpr int kMaxRanges = 50;   // 25 columns, one or two slot ranges each
+constexpr int kBuildRow = 1024;  // entries of a row in shared memory at most (a multiple of 32); longer lists are written in parts
 
-struct BuildSmem {
-    float4 cand[32];                 // staged candidates: shifted position, w = slot | compound bit
-    int rstart[kMaxRanges + 1];      // first stream index of range r; rstart[kMaxRanges] = stream length
-    int rbase[kMaxRanges];           // first cell-order position of range r
-    float rsx[kMaxRanges], rsy[kMaxRanges], rsz[kMaxRanges];   // shift of range r
+// a warp's shared memory: its ranges, then P rows of `cap` entries
+struct BuildRange {
+    float x, y, z;   // shift
+    int delta;       // cell-order position of stream index f: f + delta
 };
-
-static_assert(kGroup == 8, "the list build writes blocks of 8 entries");
-
-// candidate f of the stream (shifted position, w = slot | compound bit), or a
-// NaN sentinel past its end (fails the distance test).  r: the lane's current
-// range, advanced past the ranges that end at or before f (f only grows).
-__device__ __forceinline__ float4 fetch_cand(const PhysDev& d, const BuildSmem* sm, const float4* __restrict__ pos,
-                                             const uint32_t* __restrict__ orig, const uint32_t* __restrict__ items,
-                                             int f, int total, bool any_ex, int& r) {
-    if (f >= total) {
-        const float nan = __int_as_float(0x7fc00000);
-        return make_float4(nan, nan, nan, __uint_as_float(0u));
-    }
-    while (sm->rstart[r + 1] <= f) r++;   // rstart[kMaxRanges] = total > f
-    const int q = sm->rbase[r] + (f - sm->rstart[r]);
-    const int j = items ? (int)items[q] : q;
-    const float4 p = pos[j];
-    uint32_t tag = (uint32_t)j;
-    if (any_ex && orig[j] < (uint32_t)d.n_cp) tag |= 0x80000000u;
-    return make_float4(p.x + sm->rsx[r], p.y + sm->rsy[r], p.z + sm->rsz[r], __uint_as_float(tag));
+__host__ __device__ inline size_t build_warp_smem(int p, int cap, size_t id_bytes) {
+    return sizeof(BuildRange) * kMaxRanges + sizeof(int) * kMaxRanges + 8 + p * cap * id_bytes;
 }
 
-// The group's candidate stream (ranges set up in sm) against every member's particle.
-template <bool MIN_IMAGE>
-__device__ __forceinline__ void scan_stream(const PhysDev& d, const float4* __restrict__ pos,
-                                            const uint32_t* __restrict__ orig, const uint32_t* __restrict__ items,
-                                            BuildSmem* sm, int total, bool mine, bool any_ex, int i, float4 pi,
-                                            uint32_t oi, bool ex, int lane, int sub, int& cnt) {
-    int r = 0;
-    float4 nxt = fetch_cand(d, sm, pos, orig, items, lane, total, any_ex, r);
-    for (int t0 = 0; t0 < total; t0 += 32) {
-        __syncwarp();
-        sm->cand[lane] = nxt;
-        __syncwarp();
-        nxt = fetch_cand(d, sm, pos, orig, items, t0 + 32 + lane, total, any_ex, r);   // in flight during the tests
-        uint32_t hm = 0u;
-        if (mine) {
+// A value that is the same in every lane, in a form the compiler knows to be
+// (a warp reduction): control flow on it needs no reconvergence code around
+// the votes it holds.
+__device__ __forceinline__ int uniform(int v) { return __reduce_max_sync(0xffffffffu, v); }
+
+// One particle's hits among the warp's 32 candidates (r2 < rl2): the hit of
+// rank r stores its id j r entries past `at`, the shared address of the row's
+// next entry (nothing at or past `end`); `at` then moves past the hits.
+template <typename ID>
+__device__ __forceinline__ void append_hits(float r2, float rl2, uint32_t j, uint32_t lt, uint32_t end, uint32_t& at) {
+    if (sizeof(ID) == 2)
+        asm volatile(
+            "{\n\t.reg .pred p, q;\n\t.reg .b32 b, t;\n\t.reg .b16 h;\n\tcvt.u16.u32 h, %3;\n\tsetp.lt.f32 p, %1, %2;\n\t"
+            "vote.sync.ballot.b32 b, p, 0xffffffff;\n\tand.b32 t, b, %4;\n\tpopc.b32 t, t;\n\tmad.lo.u32 t, t, 2, %0;\n\t"
+            "setp.lt.and.u32 q, t, %5, p;\n\t@q st.shared.b16 [t], h;\n\tpopc.b32 t, b;\n\tmad.lo.u32 %0, t, 2, %0;\n\t}"
+            : "+r"(at)
+            : "f"(r2), "f"(rl2), "r"(j), "r"(lt), "r"(end)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p, q;\n\t.reg .b32 b, t;\n\tsetp.lt.f32 p, %1, %2;\n\t"
+            "vote.sync.ballot.b32 b, p, 0xffffffff;\n\tand.b32 t, b, %4;\n\tpopc.b32 t, t;\n\tmad.lo.u32 t, t, 4, %0;\n\t"
+            "setp.lt.and.u32 q, t, %5, p;\n\t@q st.shared.b32 [t], %3;\n\tpopc.b32 t, b;\n\tmad.lo.u32 %0, t, 4, %0;\n\t}"
+            : "+r"(at)
+            : "f"(r2), "f"(rl2), "r"(j), "r"(lt), "r"(end)
+            : "memory");
+}
+
+// The rows to the list: bonded exclusions out of them (in place and in order),
+// then their whole chunks, and the last partial one too if `all`.  Otherwise
+// what is left moves to the row's start.  cnt: entries in the row; done:
+// entries of the particle already in the list (a multiple of 32).
+template <typename ID, int P>
+__device__ __forceinline__ void flush_rows(const PhysDev& d, const uint32_t* __restrict__ orig, ID* rows, int cap, int i,
+                                           int base, bool all, uint32_t (&cnt)[P], uint32_t (&done)[P], int lane) {
+    __syncwarp();
+#pragma unroll 1
+    for (int p = 0; p < P; p++) {
+        if (base + p >= d.n) break;
+        const int ip = __shfl_sync(0xffffffffu, i, p);
+        uint32_t c = cnt[0], dn = done[0];
 #pragma unroll
-            for (int t = 0; t < 32 / kBuildSlices; t++) {
-                const int c = kBuildSlices * t + sub;
-                const float4 q = sm->cand[c];
-                float dx = q.x - pi.x, dy = q.y - pi.y, dz = q.z - pi.z;
-                if (MIN_IMAGE) {
-                    dx = mimg(dx, d.L, d.invL);
-                    dy = mimg(dy, d.L, d.invL);
-                    dz = mimg(dz, d.L, d.invL);
-                }
-                const bool hit = dx * dx + dy * dy + dz * dz < d.rlist2 &&
-                                 (__float_as_uint(q.w) & 0x7fffffffu) != (uint32_t)i;   // not itself
-                hm |= (hit ? 1u : 0u) << c;
+        for (int k = 1; k < P; k++) {
+            c = p == k ? cnt[k] : c;
+            dn = p == k ? done[k] : dn;
+        }
+        c = min(c, (uint32_t)cap);
+        ID* r = rows + (size_t)p * cap;
+        const uint32_t oi = d.n_cp > 0 ? orig[ip] : 0u;
+        const bool bonded = oi < (uint32_t)d.n_cp;
+        const uint32_t x0 = bonded ? d.excl_off[oi] : 0u, x1 = bonded ? d.excl_off[oi + 1] : 0u;
+        if (x1 > x0) {
+            const uint32_t n = c;
+            c = 0u;
+            for (uint32_t e0 = 0; e0 < n; e0 += 32) {
+                const uint32_t e = e0 + lane;
+                const uint32_t j = e < n ? (uint32_t)r[e] : 0u;
+                const uint32_t oj = e < n ? orig[j] : 0xffffffffu;
+                bool keep = e < n;
+                if (oj < (uint32_t)d.n_cp)
+                    for (uint32_t q = x0; q < x1; q++) keep = keep && d.excl_ids[q] != oj;
+                const unsigned kb = __ballot_sync(0xffffffffu, keep);   // (also: every lane has read its entry)
+                if (keep) r[c + __popc(kb & ((1u << lane) - 1u))] = (ID)j;
+                c += __popc(kb);
+                __syncwarp();
             }
-            if (ex)   // a compound particle drops its bonded exclusions
-                for (uint32_t b = hm; b; b &= b - 1u) {
-                    const int c = __ffs(b) - 1;
-                    const uint32_t tag = __float_as_uint(sm->cand[c].w);
-                    if ((tag >> 31) && excluded(d, oi, orig[tag & 0x7fffffffu])) hm &= ~(1u << c);
-                }
         }
-        uint32_t all = hm;   // the particle's hits (its 4 slices are lanes 4p .. 4p+3)
-        all |= __shfl_xor_sync(0xffffffffu, all, 1);
-        all |= __shfl_xor_sync(0xffffffffu, all, 2);
-        // hit of rank k goes to entry cnt + k; slice s writes ranks s, s + 4, ...
-        // (entry e of particle i at nl_word, below 2^32 because the list is
-        // smaller than 16 GB)
-        uint32_t b = all;
-        for (int k = 0; k < sub && b; k++) b &= b - 1u;
-        for (uint32_t e = (uint32_t)(cnt + sub); b; e += kBuildSlices) {
-            const int c = __ffs(b) - 1;
-            if (e < (uint32_t)d.nl_cap)
-                nl_store(d, nl_word((uint32_t)d.n_pad, (uint32_t)i, e), __float_as_uint(sm->cand[c].w) & 0x7fffffffu);
+        // lane 8 s + g writes column g of the chunks s, s + 4, ... (words past the count are never read as ids)
+        const int g = lane & 7;
+        const uint32_t chunks = all ? (c + 31u) >> 5 : c >> 5;
+        for (uint32_t q = lane >> 3; q < chunks; q += 4u) {
+            const ID* e = r + q * 32u + g;
+            const uint32_t e0 = e[0], e1 = e[8], e2 = e[16], e3 = e[24];
+            const size_t qn = (dn >> 5) + q;
+            if (qn < (size_t)(d.nl_cap >> 5)) {
+                const size_t v = (qn * d.n_pad + ip) * kGroup + g;
+                if (sizeof(ID) == 2)
+                    reinterpret_cast<uint2*>(d.nl)[v] = make_uint2(e0 | (e1 << 16), e2 | (e3 << 16));
+                else
+                    reinterpret_cast<uint4*>(d.nl)[v] = make_uint4(e0, e1, e2, e3);
+            }
+        }
+        const uint32_t whole = c & ~31u;
+        if (!all) {
+            const uint32_t e = whole + lane;
+            const ID j = e < c ? r[e] : (ID)0;
+            __syncwarp();
+            if (e < c) r[lane] = j;
+            __syncwarp();
+            dn += whole;
+            c -= whole;
+        }
 #pragma unroll
-            for (int q = 0; q < kBuildSlices; q++) b &= b - 1u;
-        }
-        cnt += __popc(all);
+        for (int k = 0; k < P; k++)
+            if (p == k) {
+                cnt[k] = c;
+                done[k] = dn;
+            }
     }
+}
+
+// The group's candidate stream (`total` of them, at least one; n_ranges ranges
+// in rg, their first stream indices in rstart) against its particles: px..
+// (NaN: not in the group) at cell-order positions first, first + 1, ...
+// ITEMS: the cell order is a list of slots.
+template <bool MIN_IMAGE, bool ITEMS, typename ID, int P>
+__device__ __forceinline__ void scan_stream(const PhysDev& d, const float4* __restrict__ pos,
+                                            const uint32_t* __restrict__ items, const BuildRange* rg, const int* rstart,
+                                            int n_ranges, int total, int first, const uint32_t* __restrict__ orig,
+                                            ID* rows, int i, uint32_t (&done)[P], const float (&px)[P],
+                                            const float (&py)[P], const float (&pz)[P], uint32_t row, uint32_t cap,
+                                            uint32_t (&cnt)[P], int lane) {
+    constexpr uint32_t kB = sizeof(ID);
+    const uint32_t lt = (1u << lane) - 1u, le = lt | (1u << lane);
+    const float rl2 = d.rlist2, nan = __int_as_float(0x7fc00000), L = d.L, invL = d.invL;
+    uint32_t at[P], end[P];
+#pragma unroll
+    for (int p = 0; p < P; p++) {
+        at[p] = row + (p * cap + cnt[p]) * kB;
+        end[p] = row + (p + 1) * cap * kB;
+    }
+    // lane l knows where ranges l and l + 32 start; a round's ranges are found
+    // from the mask of those that start inside it
+    int s0 = lane < n_ranges ? rstart[lane] : 0x3fffffff;
+    int s1 = lane + 32 < n_ranges ? rstart[lane + 32] : 0x3fffffff;
+    int f = lane, before = -1;   // the lane's stream index, the range the round starts in
+    float4 c;
+    int q;   // the candidate's cell-order position
+    auto fetch = [&]() {   // past the stream's end: its last candidate again, made to fail the test
+        const unsigned m = __reduce_or_sync(
+            0xffffffffu, ((unsigned)s0 < 32u ? 1u << s0 : 0u) | ((unsigned)s1 < 32u ? 1u << s1 : 0u));
+        const int r = before + __popc(m & le);
+        before += __popc(m);
+        s0 -= 32;
+        s1 -= 32;
+        const BuildRange g = rg[r];
+        q = min(f, total - 1) + g.delta;
+        const int j = ITEMS ? (int)__ldg(items + q) : q;
+        const float4 p = __ldg(pos + j);
+        c = make_float4(f < total ? p.x + g.x : nan, p.y + g.y, p.z + g.z, __int_as_float(j));
+        q -= first;
+        f += 32;
+    };
+    fetch();
+#pragma unroll 1
+    for (int left = total; left > 0; left -= 32) {
+        const float4 e = c;
+        const int qe = q;
+        fetch();   // in flight during the tests
+#pragma unroll
+        for (int p = 0; p < P; p++) {
+            float dx = e.x - px[p], dy = e.y - py[p], dz = e.z - pz[p];
+            if (MIN_IMAGE) {
+                dx = mimg(dx, L, invL);
+                dy = mimg(dy, L, invL);
+                dz = mimg(dz, L, invL);
+            }
+            float r2 = dx * dx + dy * dy + dz * dz;
+            r2 = qe == p ? nan : r2;   // not itself
+            append_hits<ID>(r2, rl2, __float_as_uint(e.w), lt, end[p], at[p]);
+        }
+        if (cap < (uint32_t)d.nl_cap) {   // rows shorter than the list's: to the list before one can run over
+            uint32_t room = end[0] - at[0];
+#pragma unroll
+            for (int p = 1; p < P; p++) room = min(room, end[p] - at[p]);
+            if (uniform(-(int)room) > -(int)(32u * kB)) {
+#pragma unroll
+                for (int p = 0; p < P; p++) cnt[p] = (at[p] - row) / kB - p * cap;
+                flush_rows<ID, P>(d, orig, rows, (int)cap, i, first, false, cnt, done, lane);
+#pragma unroll
+                for (int p = 0; p < P; p++) at[p] = row + (p * cap + cnt[p]) * kB;
+            }
+        }
+    }
+#pragma unroll
+    for (int p = 0; p < P; p++) cnt[p] = (at[p] - row) / kB - p * cap;
 }
 
 }  // namespace
 
-__global__ void __launch_bounds__(kBuildWarps * 32) k_build_list(PhysDev d, const float4* __restrict__ pos,
+template <typename ID, int P>
+__global__ void __launch_bounds__(kBuildWarps * 32, P == 1 ? 8 : 6) k_build_list(const __grid_constant__ PhysDev d,
+                                                                 const float4* __restrict__ pos,
                                                                  const uint32_t* __restrict__ orig,
                                                                  const uint32_t* __restrict__ items, int copy_cur,
-                                                                 int mixed) {
-    __shared__ BuildSmem s_build[kBuildWarps];
+                                                                 int mixed, int cap) {
+    extern __shared__ float4 s_build[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int pl = lane / kBuildSlices, sub = lane % kBuildSlices;
     const int gw = blockIdx.x * kBuildWarps + w;
     if (copy_cur >= 0) {   // the rebuild's copy of the permuted tmp arrays into the step arrays
         if (gw == 0 && lane == 0) *d.need_rebuild = 0;
@@ -319,56 +427,72 @@ __global__ void __launch_bounds__(kBuildWarps * 32) k_build_list(PhysDev d, cons
             d.orig_of_sorted[k] = d.orig_tmp[k];
         }
     }
-    const int base = gw * kBuildPerWarp;
+    const int base = gw * P;
     if (base >= d.n) return;   // the whole warp
-    BuildSmem* sm = &s_build[w];
-    const int qi = base + pl;   // position in the cell order
-    const bool have = qi < d.n;
+    char* smem = reinterpret_cast<char*>(s_build) + (size_t)w * build_warp_smem(P, cap, sizeof(ID));
+    BuildRange* rg = reinterpret_cast<BuildRange*>(smem);
+    int* rstart = reinterpret_cast<int*>(rg + kMaxRanges);
+    ID* rows = reinterpret_cast<ID*>(rstart + kMaxRanges + 2);   // P rows of cap entries
+    const uint32_t row = (uint32_t)__cvta_generic_to_shared(rows);
+    // lane p < P owns particle p of the warp
+    const int qi = base + lane;   // position in the cell order
+    const bool have = lane < P && qi < d.n;
     const int i = have ? (items ? (int)items[qi] : qi) : 0;   // slot
     const float4 pi = have ? pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const uint32_t oi = have ? orig[i] : 0u;
-    const bool ex = have && oi < (uint32_t)d.n_cp && d.excl_off[oi + 1] > d.excl_off[oi];
-    const bool any_ex = __any_sync(0xffffffffu, ex);
-    int cnt = 0;
+    const float nan = __int_as_float(0x7fc00000);
+    uint32_t cnt[P], done[P];
+#pragma unroll
+    for (int p = 0; p < P; p++) cnt[p] = done[p] = 0u;
+    float px[P], py[P], pz[P];
+    auto members = [&](bool in) {
+        const float x = in ? pi.x : nan;
+#pragma unroll
+        for (int p = 0; p < P; p++) {
+            px[p] = __shfl_sync(0xffffffffu, x, p);
+            py[p] = __shfl_sync(0xffffffffu, pi.y, p);
+            pz[p] = __shfl_sync(0xffffffffu, pi.z, p);
+        }
+    };
     const int m = d.m;
-
     if (m < 5) {   // one range: every particle, minimum image
         if (lane == 0) {
-            sm->rstart[0] = 0;
-            sm->rbase[0] = 0;
-            sm->rsx[0] = sm->rsy[0] = sm->rsz[0] = 0.f;
-            for (int r = 1; r <= kMaxRanges; r++) sm->rstart[r] = d.n;
+            rg[0] = BuildRange{0.f, 0.f, 0.f, 0};
+            rstart[0] = 0;
         }
         __syncwarp();
-        scan_stream<true>(d, pos, orig, items, sm, d.n, have, any_ex, i, pi, oi, ex, lane, sub, cnt);
+        members(have);
+        if (items)
+            scan_stream<true, true, ID, P>(d, pos, items, rg, rstart, 1, d.n, base, orig, rows, i, done, px, py, pz, row,
+                                           (uint32_t)cap, cnt, lane);
+        else
+            scan_stream<true, false, ID, P>(d, pos, items, rg, rstart, 1, d.n, base, orig, rows, i, done, px, py, pz, row,
+                                            (uint32_t)cap, cnt, lane);
     } else {
-        const float cs = d.L / (float)m;   // cell side
+        const float cs = d.L / (float)m, ics = (float)m / d.L;   // cell side
         int cx = -1, cy = -1, cz = 0;
         if (have) cell_xyz(d, pi, cx, cy, cz);
-        // one bit per particle, at its slice-0 lane
-        unsigned todo = __ballot_sync(0xffffffffu, have && sub == 0);
-        while (todo) {   // warp-uniform: todo is the same in every lane
+        unsigned todo = __reduce_or_sync(0xffffffffu, have ? 1u << lane : 0u);   // one bit per particle
+        while (todo) {   // warp-uniform
             const int lead = __ffs(todo) - 1;
             const int hx = __shfl_sync(0xffffffffu, cx, lead);
             const int hy = __shfl_sync(0xffffffffu, cy, lead);
             const int hz0 = __shfl_sync(0xffffffffu, cz, lead);
-            const bool mine = ((todo >> (pl * kBuildSlices)) & 1u) && cx == hx && cy == hy && cz <= hz0 + (m - 5);
-            todo &= ~__ballot_sync(0xffffffffu, mine && sub == 0);
-            int hz1 = mine ? cz : -1;   // the group's top cell
-            float bxl = mine ? pi.x : 3.4e38f, bxh = mine ? pi.x : -3.4e38f;
-            float byl = mine ? pi.y : 3.4e38f, byh = mine ? pi.y : -3.4e38f;
-            float bzl = mine ? pi.z : 3.4e38f, bzh = mine ? pi.z : -3.4e38f;
+            const bool mine = ((todo >> lane) & 1u) && cx == hx && cy == hy && cz <= hz0 + (m - 5);
+            todo &= ~__reduce_or_sync(0xffffffffu, mine ? 1u << lane : 0u);
+            const int hz1 = __reduce_max_sync(0xffffffffu, mine ? cz : -1);   // the group's top cell
+            members(mine);
+            float bxl = 3.4e38f, bxh = -3.4e38f, byl = 3.4e38f, byh = -3.4e38f, bzl = 3.4e38f, bzh = -3.4e38f;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                hz1 = max(hz1, __shfl_xor_sync(0xffffffffu, hz1, o));
-                bxl = fminf(bxl, __shfl_xor_sync(0xffffffffu, bxl, o));
-                bxh = fmaxf(bxh, __shfl_xor_sync(0xffffffffu, bxh, o));
-                byl = fminf(byl, __shfl_xor_sync(0xffffffffu, byl, o));
-                byh = fmaxf(byh, __shfl_xor_sync(0xffffffffu, byh, o));
-                bzl = fminf(bzl, __shfl_xor_sync(0xffffffffu, bzl, o));
-                bzh = fmaxf(bzh, __shfl_xor_sync(0xffffffffu, bzh, o));
+            for (int p = 0; p < P; p++) {   // a NaN x marks a particle outside the group
+                const bool in = px[p] == px[p];
+                bxl = fminf(bxl, px[p]);
+                bxh = fmaxf(bxh, px[p]);
+                byl = in ? fminf(byl, py[p]) : byl;
+                byh = in ? fmaxf(byh, py[p]) : byh;
+                bzl = in ? fminf(bzl, pz[p]) : bzl;
+                bzh = in ? fmaxf(bzh, pz[p]) : bzh;
             }
-            // lane c < 25: column (hx + c / 5 - 2, hy + c % 5 - 2), ranges 2c and 2c + 1
+            // lane c < 25: column (hx + c / 5 - 2, hy + c % 5 - 2), one or two ranges
             int b0 = 0, l0 = 0, b1 = 0, l1 = 0;
             float sx = 0.f, sy = 0.f, sz0 = 0.f, sz1 = 0.f;
             if (lane < 25) {
@@ -384,10 +508,11 @@ __global__ void __launch_bounds__(kBuildWarps * 32) k_build_list(PhysDev d, cons
                     if (y < 0) { y += m; sy = -d.L; } else if (y >= m) { y -= m; sy = d.L; }
                     const int col = (x * m + y) * m;
                     // cells within the reach of the group's z-range (unwrapped; at
-                    // most m of them: the group spans <= m - 4 cells)
+                    // most m of them: the group spans <= m - 4 cells).  Both ends
+                    // clamped: a position far outside the box stays inside cstart.
                     const float reach = sqrtf(fmaxf(d.rlist2 - g2, 0.f)) + 1e-4f * cs;
-                    const int u0 = max((int)floorf((bzl - reach) / cs), hz0 - 2);
-                    const int u1 = min((int)floorf((bzh + reach) / cs), hz1 + 2);
+                    const int u0 = min(max((int)floorf((bzl - reach) * ics), hz0 - 2), hz1 + 2);
+                    const int u1 = max(min((int)floorf((bzh + reach) * ics), hz1 + 2), u0 - 1);
                     if (u0 < 0) {
                         b0 = (int)d.cstart[col + u0 + m];
                         l0 = (int)d.cstart[col + m] - b0;
@@ -406,7 +531,7 @@ __global__ void __launch_bounds__(kBuildWarps * 32) k_build_list(PhysDev d, cons
                     }
                 }
             }
-            // stream offsets: inclusive scan of the per-column lengths
+            // stream offsets: inclusive scan of the per-column lengths; the non-empty ranges in column order
             const int len = l0 + l1;
             int incl = len;
 #pragma unroll
@@ -414,31 +539,43 @@ __global__ void __launch_bounds__(kBuildWarps * 32) k_build_list(PhysDev d, cons
                 const int y = __shfl_up_sync(0xffffffffu, incl, o);
                 if (lane >= o) incl += y;
             }
-            const int total = __shfl_sync(0xffffffffu, incl, 31);
-            __syncwarp();   // the previous group's readers of sm are done
-            if (lane < 25) {
-                const int st = incl - len;
-                sm->rstart[2 * lane] = st;
-                sm->rstart[2 * lane + 1] = st + l0;
-                sm->rbase[2 * lane] = b0;
-                sm->rbase[2 * lane + 1] = b1;
-                sm->rsx[2 * lane] = sm->rsx[2 * lane + 1] = sx;
-                sm->rsy[2 * lane] = sm->rsy[2 * lane + 1] = sy;
-                sm->rsz[2 * lane] = sz0;
-                sm->rsz[2 * lane + 1] = sz1;
+            const int total = uniform(incl);
+            const unsigned has0 = __ballot_sync(0xffffffffu, l0 > 0), has1 = __ballot_sync(0xffffffffu, l1 > 0);
+            const unsigned lt = (1u << lane) - 1u;
+            int at = __popc(has0 & lt) + __popc(has1 & lt);
+            __syncwarp();   // the previous group's readers are done
+            const int st = incl - len;
+            if (l0 > 0) {
+                rg[at] = BuildRange{sx, sy, sz0, b0 - st};
+                rstart[at++] = st;
             }
-            if (lane == 0) sm->rstart[kMaxRanges] = total;
+            if (l1 > 0) {
+                rg[at] = BuildRange{sx, sy, sz1, b1 - st - l0};
+                rstart[at] = st + l0;
+            }
             __syncwarp();
-            scan_stream<false>(d, pos, orig, items, sm, total, mine, any_ex, i, pi, oi, ex, lane, sub, cnt);
+            const int n_ranges = __popc(has0) + __popc(has1);
+            if (items)
+                scan_stream<false, true, ID, P>(d, pos, items, rg, rstart, n_ranges, total, base, orig, rows, i, done, px,
+                                                py, pz, row, (uint32_t)cap, cnt, lane);
+            else
+                scan_stream<false, false, ID, P>(d, pos, items, rg, rstart, n_ranges, total, base, orig, rows, i, done,
+                                                 px, py, pz, row, (uint32_t)cap, cnt, lane);
         }
     }
-    if (have && sub == 0) {
-        d.nl_cnt[i] = (uint32_t)min(cnt, d.nl_cap);
-        if (cnt > d.nl_cap) {
-            atomicOr(d.err, ERR_BIT_PHYS_LIST_OVERFLOW);
-            atomicMax(d.nl_need, cnt);
+    uint32_t found[P];   // before the exclusions: what a row may have run over the list's capacity by
+#pragma unroll
+    for (int p = 0; p < P; p++) found[p] = done[p] + cnt[p];
+    flush_rows<ID, P>(d, orig, rows, cap, i, base, true, cnt, done, lane);
+#pragma unroll
+    for (int p = 0; p < P; p++)
+        if (lane == p && have) {
+            d.nl_cnt[i] = min(done[p] + cnt[p], (uint32_t)d.nl_cap);
+            if (found[p] > (uint32_t)d.nl_cap) {
+                atomicOr(d.err, ERR_BIT_PHYS_LIST_OVERFLOW);
+                atomicMax(d.nl_need, (int)found[p]);
+            }
         }
-    }
 }
 
 // ------------------------------------------------------------- bonded terms ---
@@ -1209,11 +1346,30 @@ void launch_set_xref(const PhysDev& d, const float4* pos, cudaStream_t s) {
 
 bool list_ids_16bit(int n_pad) { return !kStagedList && n_pad <= 65536; }
 
+namespace {
+template <typename ID, int P>
+void build_list(const PhysDev& d, const float4* pos, const uint32_t* orig, const uint32_t* items, int copy_cur,
+                bool mixed, cudaStream_t s) {
+    const int warps = (d.n + P - 1) / P;
+    const int cap = std::min(d.nl_cap, kBuildRow);
+    const size_t smem = kBuildWarps * build_warp_smem(P, cap, sizeof(ID));
+    if (smem > 48 * 1024)
+        cudaFuncSetAttribute(k_build_list<ID, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_build_list<ID, P><<<(warps + kBuildWarps - 1) / kBuildWarps, kBuildWarps * 32, smem, s>>>(
+        d, pos, orig, items, copy_cur, mixed ? 1 : 0, cap);
+}
+}  // namespace
+
 void launch_build_list(const PhysDev& d, const float4* pos, const uint32_t* orig, const uint32_t* items, int copy_cur,
                        bool mixed, cudaStream_t s) {
-    const int warps = (d.n + 7) / 8;   // 8 particles per warp
-    k_build_list<<<(warps + kBuildWarps - 1) / kBuildWarps, kBuildWarps * 32, 0, s>>>(d, pos, orig, items, copy_cur,
-                                                                                    mixed ? 1 : 0);
+    // (measured at kBuildOneBelow)
+    if (d.n < kBuildOneBelow) {
+        if (d.nl16) build_list<uint16_t, 1>(d, pos, orig, items, copy_cur, mixed, s);
+        else build_list<uint32_t, 1>(d, pos, orig, items, copy_cur, mixed, s);
+    } else {
+        if (d.nl16) build_list<uint16_t, 4>(d, pos, orig, items, copy_cur, mixed, s);
+        else build_list<uint32_t, 4>(d, pos, orig, items, copy_cur, mixed, s);
+    }
 }
 
 namespace {

@@ -9,7 +9,13 @@ namespace lima {
 
 constexpr int kTB = 256;         // threads per block of the per-particle kernels and the step kernel
 constexpr int kGroup = 8;        // lanes per particle in the list and step kernels
-constexpr int kBuildWarps = 4;   // warps per block of the list build (8 particles per warp)
+constexpr int kBuildWarps = 4;   // warps per block of the list build
+// The list build gives a warp one particle below this box size (more warps,
+// shorter streams) and four from it on (fewer tests and one stream's fetches
+// for four).  A host-issued rebuild with 1 / 4 particles a warp: 4,096
+// particles 61 / 72 us, 8,192 76 / 78, 32,024 136 / 124, 258,192 748 / 571
+// (14 us of each the call's synchronisation).
+constexpr int kBuildOneBelow = 16384;
 constexpr int kMaxTypes = 32;    // LIMA_MAX_ATOM_TYPES
 constexpr int kScanThreads = 1024;
 

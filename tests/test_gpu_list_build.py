@@ -1,0 +1,69 @@
+"""The Verlet-list build over its variants: one and four particles a warp, 16-
+and 32-bit ids, boxes of fewer than five cells a side (minimum image), rows
+longer than the build keeps in shared memory, bonded exclusions, partial last
+chunks.  The list read back has to hold every pair within the list radius that
+a brute-force search finds, none twice, no pair beyond it and no excluded one.
+Distances within 2e-6 nm of the radius (FP32 coordinates of a box of at most
+14 nm round at 1e-6 nm) may fall on either side."""
+import numpy as np
+import pytest
+
+from quantom_b200 import engine as E
+from quantom_b200 import systems as S
+
+pytestmark = pytest.mark.gpu
+
+# box, waters, chains, length, cutoff
+CASES = [(2.7, 601, 0, 0, 1.2),        # two cells a side
+         (3.0, 879, 0, 0, 1.2),        # four
+         (3.3, 1100, 0, 0, 1.2),       # five: the smallest grid that is walked
+         (4.0, 1901, 2, 23, 1.2),      # exclusions
+         (4.4, 2600, 2, 24, 2.05),     # rows of 1,300 entries, minimum image
+         (5.6, 5500, 3, 30, 2.05),     # rows of 1,300 entries in the grid
+         (8.1, 16385, 4, 50, 1.0),     # four particles a warp, an odd count
+         (8.1, 16385, 4, 50, 2.05),    # the same with long rows
+         (13.0, 66003, 2, 64, 1.0)]    # 32-bit ids
+
+
+@pytest.mark.parametrize("box,waters,chains,length,cutoff", CASES)
+def test_list_is_the_brute_force_list(box, waters, chains, length, cutoff):
+    import torch
+    spec = S.SystemSpec("box", box, waters, cutoff=cutoff, chains=S.ChainSpec(chains, length) if chains else None,
+                        mc_sweeps=4)
+    s = S.make_system(spec, seed=11)
+    skin = 0.05
+    p = E.default_params(box_len=box, cutoff=cutoff, dt=spec.dt, semantics=E.SEMANTICS_PHYSICS, skin=skin,
+                         switch_on=cutoff - 0.2, nlist_period=0)
+    with E.Engine(s, p) as eng:
+        off, ids = eng.nlist(E.NL_PAIR)
+        fc, fs = eng.positions()
+    n_of = s.compounds["n_particles"] if chains else []
+    x = np.concatenate([fc[c, :k] for c, k in enumerate(n_of)] + [fs]).astype(np.float64)
+    x -= np.floor(x / box) * box
+    base = np.concatenate([[0], np.cumsum(n_of)]).astype(int)
+    excl = {(base[c] + q, base[ig["compound_ids"][z]] + ig["local_ids"][z])
+            for c, k in enumerate(n_of) for q in range(k) for ig in [s.compounds[c]["lj_ignore_list"][q]]
+            for z in range(ig["n_ignores"])}
+    n, r = len(x), cutoff + skin
+    got = np.zeros((2, len(ids)), np.int64)
+    got[0], got[1] = np.repeat(np.arange(n), np.diff(off)), ids
+    keys = np.sort(got[0] * n + got[1])
+    assert (np.diff(keys) > 0).all()
+    assert not any(i * n + j in set(keys[np.searchsorted(keys, i * n):np.searchsorted(keys, (i + 1) * n)])
+                   for i, j in excl)
+    xt = torch.as_tensor(x, device="cuda")
+    keys = torch.as_tensor(keys, device="cuda")
+    ex = torch.as_tensor(sorted(int(i) * n + int(j) for i, j in excl), dtype=torch.int64, device="cuda")
+    for lo in range(0, n, 512):
+        d = xt[None, :, :] - xt[lo: lo + 512, None, :]
+        d -= box * torch.round(d / box)
+        dist = d.norm(dim=-1)
+        rows = torch.arange(lo, min(n, lo + 512), device="cuda")
+        dist[rows - lo, rows] = 1e9
+        a, b = int(torch.searchsorted(keys, lo * n)), int(torch.searchsorted(keys, min(n, lo + 512) * n))
+        mine = keys[a:b]
+        assert (dist.reshape(-1)[mine - lo * n] < r + 2e-6).all()
+        want = torch.nonzero(dist < r - 2e-6)
+        want = (want[:, 0] + lo) * n + want[:, 1]
+        want = want[~torch.isin(want, ex)]
+        assert torch.isin(want, mine).all()
