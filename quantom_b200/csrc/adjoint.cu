@@ -33,14 +33,6 @@ constexpr int kListEpoch = 10;
 
 __device__ __forceinline__ float mimg_a(float d, float L, float invL) { return d - L * rintf(d * invL); }
 
-// Minimum image of a difference of two coordinates in [0, L): the rounding of
-// d / L (|d / L| < 1) by adding and subtracting 1.5 * 2^23, three operations of
-// the FP32 pipes (rintf takes a slower one).
-__device__ __forceinline__ float mimg_add(float d, float L, float invL) {
-    const float k = fmaf(d, invL, 12582912.f) - 12582912.f;
-    return fmaf(-L, k, d);
-}
-
 // 1 / x to about half an ulp: the special-function unit's reciprocal and one
 // Newton step (x positive, far from the denormal and overflow ranges)
 __device__ __forceinline__ float rcp_newton(float x) {

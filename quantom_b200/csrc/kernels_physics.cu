@@ -35,8 +35,6 @@
 namespace lima {
 namespace {
 
-constexpr double kR = 8.314462618;   // J/(mol K)
-
 // error-free sum: s + e == a + b exactly
 __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
     s = a + b;
@@ -809,6 +807,8 @@ __device__ __forceinline__ void finish_sums(const PhysDev& d, int slot, cudaGrap
     __syncthreads();
     if (!s_last) return;
     __threadfence();
+    // (read beside the partials; the block that finished last sees every block's request)
+    const int due = TAIL && INTEGRATE && threadIdx.x == 0 ? *(volatile int*)d.need_rebuild : 0;
     double a[kRed];
 #pragma unroll
     for (int q = 0; q < nq; q++) a[q] = 0.0;
@@ -827,7 +827,7 @@ __device__ __forceinline__ void finish_sums(const PhysDev& d, int slot, cudaGrap
     for (int q = 0; q < nq; q++)
         for (int k = 0; k < kTB / 32; k++) tot[q] += s_red[k][q];
     const double kin = tot[0];
-    const double temp = 2.0 * kin / (3.0 * (double)d.n * kR);
+    const double temp = kin * d.temp_of_kin;
     d.e_last[LIMA_E_KINETIC] = kin;
     d.e_last[LIMA_E_TEMPERATURE] = temp;
     if (ENERGY) {
@@ -848,11 +848,11 @@ __device__ __forceinline__ void finish_sums(const PhysDev& d, int slot, cudaGrap
     if (slot < 2) {
         float lam = 1.f;
         if (d.thermostat == LIMA_THERMOSTAT_BERENDSEN && temp > 0.0)
-            lam = (float)sqrt(1.0 + d.dt / d.tau_t * (d.t_target / temp - 1.0));
+            lam = (float)sqrt(1.0 + d.dt_tau * (d.t_target / temp - 1.0));
         d.lambda[slot ^ 1] = lam;
     }
     *d.done = 0u;   // for the next launch
-    if (TAIL && INTEGRATE && tail != nullptr && *(volatile int*)d.need_rebuild) {
+    if (TAIL && INTEGRATE && tail != nullptr && due) {
         if (cudaGraphLaunch(tail, cudaStreamGraphTailLaunch) == cudaSuccess)
             *d.rebuild_count += 1ull;
         else
@@ -1114,6 +1114,7 @@ __device__ __forceinline__ void step_body(const PhysDev& d, int cur, int slot, c
         case 0: LIMA_ROWS_CALL(0); break;
         case 1: LIMA_ROWS_CALL(1); break;
         case 2: LIMA_ROWS_CALL(2); break;
+        case 3: LIMA_ROWS_CALL(3); break;
         case 4: LIMA_ROWS_CALL(4); break;
         default: LIMA_ROWS_CALL(7); break;
     }

@@ -66,6 +66,7 @@ struct PhysDev {
     int precision;      // lima_precision
     int thermostat;     // lima_thermostat
     double t_target, tau_t;
+    double temp_of_kin, dt_tau;   // 2 / (3 n R), dt / tau_t
     int n_types;
     float4* pos[2];
     float4* vel;

@@ -167,6 +167,8 @@ int phys_setup(const PhysHost& h, PhysDev& d, cudaStream_t s, std::vector<void*>
     d.thermostat = p.thermostat;
     d.t_target = p.t_target;
     d.tau_t = p.tau_t;
+    d.temp_of_kin = 2.0 / (3.0 * (double)d.n * 8.314462618);   // J/(mol K)
+    d.dt_tau = p.dt / p.tau_t;
 
     // types and the Lorentz-Berthelot table (sigma^2, 4 eps)
     int max_type = 0;
