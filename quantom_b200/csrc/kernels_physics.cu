@@ -889,9 +889,11 @@ struct ChunkIds<uint32_t> {
     }
 };
 
-// One lane's entries of its particle's Verlet list: `rows` entries, four per
-// chunk column (col: the lane's column of chunk 0; cstride: vectors between
-// chunks), each chunk one vector load and four position gathers in flight.
+// One lane's entries of its particle's Verlet list: column g of every H-th
+// 32-entry chunk, n_full whole chunks and, if tail, `tail` entries of the
+// partial last one; four entries per chunk column (col: the lane's column of
+// its first chunk; cstride: vectors between its chunks), each chunk one vector
+// load and four position gathers in flight.
 // In the last, partial chunk the words past the lane's count are not ids
 // (the gathers for them re-read the first entry and are not evaluated).
 // MIXED: compensated sums every two chunks (8 pairs).  WM: the axes that take
@@ -900,11 +902,10 @@ struct ChunkIds<uint32_t> {
 // registers to spare for it).
 template <bool MIXED, bool ENERGY, bool SWITCH, int WM, typename ID>
 __device__ __forceinline__ void pair_rows(const PhysDev& d, const float2* row, float4 pi, const float4* __restrict__ pos,
-                                          const typename ChunkIds<ID>::V* __restrict__ col, uint32_t cstride, int rows,
-                                          float& fx, float& fy, float& fz, float& cxx, float& cyy, float& czz,
+                                          const typename ChunkIds<ID>::V* __restrict__ col, uint32_t cstride, int full,
+                                          int tail, float& fx, float& fy, float& fz, float& cxx, float& cyy, float& czz,
                                           float& e_i, float& w_i) {
     constexpr bool kAhead = !MIXED && (SWITCH || !ENERGY);
-    const int full = rows >> 2, tail = rows & 3;
     const int nch = full + (tail ? 1 : 0);
     uint32_t off = 0;
     int c = 0;
@@ -1018,7 +1019,7 @@ __device__ __forceinline__ void pair_walk_staged(const PhysDev& d, const float2*
         mbar_init_fence();
     }
     __syncthreads();
-    if (active && threadIdx.x % kStepLanes == 0) atomicMax(&s_rows, rows);
+    if (active && threadIdx.x % kGroup == 0) atomicMax(&s_rows, rows);
     __syncthreads();
     const int bchunks = (s_rows + 3) / 4;
     const int nst = (bchunks + kStageChunks - 1) / kStageChunks;
@@ -1064,7 +1065,9 @@ __device__ __forceinline__ void pair_walk_staged(const PhysDev& d, const float2*
 }
 #endif  // LIMA_STAGED_LIST
 
-template <bool MIXED, bool ENERGY, bool INTEGRATE, bool SWITCH, bool TAIL, typename ID>
+// LPP lanes walk one particle's list: lane g + 8 h takes column g of the chunks
+// h, h + LPP / 8, ...
+template <int LPP, bool MIXED, bool ENERGY, bool INTEGRATE, bool SWITCH, bool TAIL, typename ID>
 __device__ __forceinline__ void step_body(const PhysDev& d, int cur, int slot, cudaGraphExec_t tail) {
     // the LJ table as lj_pair_step reads it: (sigma^2, 24 eps)
     extern __shared__ float2 s_tab[];
@@ -1074,8 +1077,8 @@ __device__ __forceinline__ void step_body(const PhysDev& d, int cur, int slot, c
         s_tab[q] = make_float2(t.x, 6.f * t.y);
     }
     __syncthreads();
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / kStepLanes;
-    const int g = threadIdx.x % kStepLanes;
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / LPP;
+    const int lp = threadIdx.x % LPP, g = lp % kGroup, h = lp / kGroup;
     const bool active = i < d.n;
     // FP64 sums of this thread: kinetic energy, LJ energy, LJ virial
     double red[kRed] = {0.0, 0.0, 0.0};
@@ -1085,31 +1088,38 @@ __device__ __forceinline__ void step_body(const PhysDev& d, int cur, int slot, c
     float fx = 0.f, fy = 0.f, fz = 0.f, cxx = 0.f, cyy = 0.f, czz = 0.f;
     float e_i = 0.f, w_i = 0.f;
     const int cnt = active ? (int)d.nl_cnt[i] : 0;
-    // this lane's entries: g, g + 8, g + 16, ... below cnt
-    const int rows = cnt > g ? (cnt - g + kStepLanes - 1) / kStepLanes : 0;
     // the axes that take the minimum image: those on which some particle of the
     // warp lies within r_c of a face (one axis alone, or all three)
     const unsigned wm = __reduce_or_sync(0xffffffffu, active ? face_axes(d, pi) : 0u);
 #if LIMA_STAGED_LIST
+    const int rows = cnt > g ? (cnt - g + kGroup - 1) / kGroup : 0;   // this lane's entries: g, g + 8, ... below cnt
+    (void)h;
     pair_walk_staged<MIXED, ENERGY, SWITCH>(d, row, pi, pos, rows, active, wm, fx, fy, fz, cxx, cyy, czz, e_i, w_i);
 #else
     // the lane's column of chunk 0 (nl_word with k = g), chunks n_pad * 8 vectors apart
     using V = typename ChunkIds<ID>::V;
-    const V* __restrict__ col = reinterpret_cast<const V*>(d.nl) + (uint32_t)i * kGroup + g;
-    const uint32_t cstride = (uint32_t)d.n_pad * kGroup;
-    {   // the warp's list chunks into L2 at once: chunk q of its 4 particles is
-        // 4 x 32 contiguous ids, one bulk prefetch per lane q (no completion to wait for)
-        const int wch = ((int)__reduce_max_sync(0xffffffffu, (unsigned)rows) + 3) / 4;
+    constexpr int H = LPP / kGroup;
+    const uint32_t chunk = (uint32_t)d.n_pad * kGroup, cstride = H * chunk;
+    const V* __restrict__ col = reinterpret_cast<const V*>(d.nl) + (uint32_t)i * kGroup + g + h * chunk;
+    // this lane's chunks with four entries (whole ones, and the partial last one where it reaches
+    // that far), then its 0 .. 3 entries of the last
+    const int whole = cnt / kListChunk;
+    const int last = whole % H == h ? max((cnt - whole * kListChunk - g + kGroup - 1) / kGroup, 0) : 0;
+    const int full = (whole - h + H - 1) / H + (last >> 2), part = last & 3;
+    {   // the warp's list chunks into L2 at once: chunk q of its 32 / LPP particles is
+        // as many times 32 contiguous ids, one bulk prefetch per lane q (no completion to wait for)
+        const int wch = ((int)__reduce_max_sync(0xffffffffu, (unsigned)cnt) + kListChunk - 1) / kListChunk;
         const int lane = threadIdx.x & 31;
         if (lane < wch) {
-            const uint32_t i0 = (blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) / kStepLanes;
+            const uint32_t i0 = (blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) / LPP;
             const char* a = reinterpret_cast<const char*>(d.nl) + ((size_t)lane * d.n_pad + i0) * kListChunk * sizeof(ID);
-            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"((unsigned)(4 * kListChunk * sizeof(ID)))
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"((unsigned)(32 / LPP * kListChunk * sizeof(ID)))
                          : "memory");
         }
     }
 #define LIMA_ROWS_CALL(WM) \
-    pair_rows<MIXED, ENERGY, SWITCH, WM, ID>(d, row, pi, pos, col, cstride, rows, fx, fy, fz, cxx, cyy, czz, e_i, w_i)
+    pair_rows<MIXED, ENERGY, SWITCH, WM, ID>(d, row, pi, pos, col, cstride, full, part, fx, fy, fz, cxx, cyy, czz, e_i, \
+                                             w_i)
     switch (wm) {
         case 0: LIMA_ROWS_CALL(0); break;
         case 1: LIMA_ROWS_CALL(1); break;
@@ -1120,9 +1130,9 @@ __device__ __forceinline__ void step_body(const PhysDev& d, int cur, int slot, c
     }
 #undef LIMA_ROWS_CALL
 #endif
-    // reduce the kStepLanes lanes of this particle (warp shuffles)
+    // reduce the LPP lanes of this particle (warp shuffles)
 #pragma unroll
-    for (int o = kStepLanes / 2; o > 0; o >>= 1) {
+    for (int o = LPP / 2; o > 0; o >>= 1) {
         if (MIXED) {
             const float ox = __shfl_xor_sync(0xffffffffu, fx, o), oy = __shfl_xor_sync(0xffffffffu, fy, o),
                         oz = __shfl_xor_sync(0xffffffffu, fz, o);
@@ -1143,7 +1153,7 @@ __device__ __forceinline__ void step_body(const PhysDev& d, int cur, int slot, c
         }
     }
     const uint32_t oi = active ? d.orig_of_sorted[i] : 0xffffffffu;
-    if (active && g == 0) {
+    if (active && lp == 0) {
         float e_b = 0.f;
         if (oi < (uint32_t)d.n_cp) {
             // the bonded kernel's forces on this particle (it runs beside this
@@ -1268,26 +1278,37 @@ __device__ __forceinline__ void step_body(const PhysDev& d, int cur, int slot, c
 // FP32: at most 48 registers, 5 blocks of 256 per SM.  Mixed keeps the
 // compiler's own choice (a 5-block bound slowed it).
 // ID: the list's slot-id type (uint16_t when the slots fit, else uint32_t).
-template <bool ENERGY, bool INTEGRATE, bool SWITCH, bool TAIL, typename ID>
+template <int LPP, bool ENERGY, bool INTEGRATE, bool SWITCH, bool TAIL, typename ID>
 __global__ void __launch_bounds__(kTB, 5) k_step(PhysDev d, int cur, int slot, cudaGraphExec_t tail) {
-    step_body<false, ENERGY, INTEGRATE, SWITCH, TAIL, ID>(d, cur, slot, tail);
+    step_body<LPP, false, ENERGY, INTEGRATE, SWITCH, TAIL, ID>(d, cur, slot, tail);
 }
-template <bool ENERGY, bool INTEGRATE, bool SWITCH, bool TAIL, typename ID>
+template <int LPP, bool ENERGY, bool INTEGRATE, bool SWITCH, bool TAIL, typename ID>
 __global__ void __launch_bounds__(kTB) k_step_mixed(PhysDev d, int cur, int slot, cudaGraphExec_t tail) {
-    step_body<true, ENERGY, INTEGRATE, SWITCH, TAIL, ID>(d, cur, slot, tail);
+    step_body<LPP, true, ENERGY, INTEGRATE, SWITCH, TAIL, ID>(d, cur, slot, tail);
 }
 
 // ---------------------------------------------------------------- launchers --
+int step_lanes(const PhysDev& d, bool energy) {
+    if (kStagedList) return kGroup;
+    if (energy) return d.n < kStepEnergy32Below ? 32 : kGroup;
+    return d.n < kStep32Below ? 32 : (d.n < kStep16Below ? 16 : kGroup);
+}
+
+// the n_pad slots' lanes
+int step_blocks(const PhysDev& d, bool energy) {
+    return (int)(((size_t)d.n_pad * step_lanes(d, energy) + kTB - 1) / kTB);
+}
+
 namespace {
 
 // The step kernel with a programmatic dependency on the kernel before it in
 // the stream (the bonded kernel): it may start before that one has finished
 // and waits for it only where it reads its results.
 template <typename K>
-void launch_programmatic(K kernel, const PhysDev& d, int cur, int slot, cudaGraphExec_t tail, size_t smem,
+void launch_programmatic(K kernel, const PhysDev& d, int blocks, int cur, int slot, cudaGraphExec_t tail, size_t smem,
                          cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)step_blocks(d));
+    cfg.gridDim = dim3((unsigned)blocks);
     cfg.blockDim = dim3(kTB);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
@@ -1299,17 +1320,29 @@ void launch_programmatic(K kernel, const PhysDev& d, int cur, int slot, cudaGrap
     cudaLaunchKernelEx(&cfg, kernel, d, cur, slot, tail);
 }
 
+template <int LPP, bool MIXED, bool ENERGY, bool INTEGRATE, bool TAIL, typename ID>
+void step_variant_lanes(const PhysDev& d, int cur, int slot, cudaGraphExec_t tail, cudaStream_t s) {
+    const size_t smem = sizeof(float2) * d.n_types * d.n_types;
+    const int blocks = step_blocks(d, ENERGY);
+    if (MIXED && d.use_switch)
+        launch_programmatic(k_step_mixed<LPP, ENERGY, INTEGRATE, true, TAIL, ID>, d, blocks, cur, slot, tail, smem, s);
+    else if (MIXED)
+        launch_programmatic(k_step_mixed<LPP, ENERGY, INTEGRATE, false, TAIL, ID>, d, blocks, cur, slot, tail, smem, s);
+    else if (d.use_switch)
+        launch_programmatic(k_step<LPP, ENERGY, INTEGRATE, true, TAIL, ID>, d, blocks, cur, slot, tail, smem, s);
+    else
+        launch_programmatic(k_step<LPP, ENERGY, INTEGRATE, false, TAIL, ID>, d, blocks, cur, slot, tail, smem, s);
+}
+
 template <bool MIXED, bool ENERGY, bool INTEGRATE, bool TAIL, typename ID>
 void step_variant_id(const PhysDev& d, int cur, int slot, cudaGraphExec_t tail, cudaStream_t s) {
-    const size_t smem = sizeof(float2) * d.n_types * d.n_types;
-    if (MIXED && d.use_switch)
-        launch_programmatic(k_step_mixed<ENERGY, INTEGRATE, true, TAIL, ID>, d, cur, slot, tail, smem, s);
-    else if (MIXED)
-        launch_programmatic(k_step_mixed<ENERGY, INTEGRATE, false, TAIL, ID>, d, cur, slot, tail, smem, s);
-    else if (d.use_switch)
-        launch_programmatic(k_step<ENERGY, INTEGRATE, true, TAIL, ID>, d, cur, slot, tail, smem, s);
-    else
-        launch_programmatic(k_step<ENERGY, INTEGRATE, false, TAIL, ID>, d, cur, slot, tail, smem, s);
+    switch (step_lanes(d, ENERGY)) {
+#if !LIMA_STAGED_LIST
+        case 32: step_variant_lanes<32, MIXED, ENERGY, INTEGRATE, TAIL, ID>(d, cur, slot, tail, s); break;
+        case 16: step_variant_lanes<16, MIXED, ENERGY, INTEGRATE, TAIL, ID>(d, cur, slot, tail, s); break;
+#endif
+        default: step_variant_lanes<8, MIXED, ENERGY, INTEGRATE, TAIL, ID>(d, cur, slot, tail, s); break;
+    }
 }
 
 template <bool MIXED, bool ENERGY, bool INTEGRATE, bool TAIL>

@@ -346,7 +346,7 @@ int phys_setup(const PhysHost& h, PhysDev& d, cudaStream_t s, std::vector<void*>
         d.nl_cnt = a.take<uint32_t>(d.n_pad);
         d.nl_need = a.take<int>(1);
         d.term_force = a.take<float4>(d.n_term_slots);
-        d.part = a.take<double>((size_t)step_blocks(d) * kRedStride);
+        d.part = a.take<double>((size_t)std::max(step_blocks(d, false), step_blocks(d, true)) * kRedStride);
         d.bpart = a.take<double>((size_t)bonded_blocks(d) * 4);
         d.done = a.take<unsigned int>(1);
         d.e_last = a.take<double>(LIMA_E_COUNT);

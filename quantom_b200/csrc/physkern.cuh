@@ -19,9 +19,14 @@ constexpr int kBuildOneBelow = 16384;
 constexpr int kMaxTypes = 32;    // LIMA_MAX_ATOM_TYPES
 constexpr int kScanThreads = 1024;
 
-// lanes per particle in the step kernel: one list column each
-constexpr int kStepLanes = 8;
-static_assert(kStepLanes == kGroup, "the step kernel gives each lane one list column");
+// Lanes per particle in the step kernel: 8 (one list column each), more in
+// boxes too small to fill the SMs' warps, where a lane's chain of chunk loads
+// and gathers is the time.  Per step with 8 / 16 / 32 lanes: 880 particles
+// 16.3 / 15.0 / 14.2 us, 1,948 17.5 / 16.3 / 15.8, 4,096 18.3 / 16.6 / 18.6,
+// 8,192 20.1 / 21.4 / 23.1.  With energies (more sums to reduce, and the frame
+// behind it) 200 steps: 880 4.60 / 4.52 / 3.97 ms, 1,948 4.72 / 5.11 / 5.09,
+// 3,893 4.99 / 5.11 / 5.77.
+constexpr int kStep32Below = 2048, kStep16Below = 6144, kStepEnergy32Below = 1024;
 // the step kernel reads its list rows from shared memory, staged by bulk
 // copies in groups of kStageRows rows (false: per-lane loads from the list).
 // Built into liblima_b200_staged.so (LIMA_STAGED_LIST=1) beside the default
@@ -61,10 +66,9 @@ bool list_ids_16bit(int n_pad);
 // bytes of one list entry
 __host__ __device__ inline size_t nl_entry_bytes(const PhysDev& d) { return d.nl16 ? 2 : 4; }
 
-// blocks of the step kernel (kStepLanes lanes per particle slot, n_pad a multiple of 32)
-__host__ __device__ inline int step_blocks(const PhysDev& d) {
-    return (int)(((size_t)d.n_pad * kStepLanes + kTB - 1) / kTB);
-}
+// lanes that walk one particle's list in the step kernel, and its blocks
+int step_lanes(const PhysDev& d, bool energy);
+int step_blocks(const PhysDev& d, bool energy);
 // blocks of the bonded kernel (one thread per term)
 __host__ __device__ inline int bonded_blocks(const PhysDev& d) {
     const int nt = d.n_bonds + d.n_angles + d.n_dih;
