@@ -85,6 +85,7 @@ struct lima_ctx {
     lima::FrameLog log;        // physics: frames recorded every log.every steps
     // physics readbacks: device copies of the reference's state structs (pool)
     void* read_stage = nullptr;
+    int* err_word = nullptr;   // pinned: the device's error word of the last synchronisation
     lima::RenderBuf render;    // headless rasterizer buffers (allocated by the first lima_render)
 
     template <typename T>
@@ -105,6 +106,7 @@ struct lima_ctx {
         for (void* ptr : dallocs) cudaFree(ptr);
         for (void* ptr : pool_allocs) lima::pool_free(ptr, stream);
         if (!pool_allocs.empty()) cudaStreamSynchronize(stream);
+        lima::pinned_free(err_word);
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
         if (fork.fork) cudaEventDestroy(fork.fork);
@@ -384,11 +386,19 @@ void phys_launch_step(lima_ctx* c, int parity) {
     c->graph_kernels = lima::phys_step_kernels(c->phys, parity, c->stream);
 }
 
-void check_device_errors(lima_ctx* c) {
+// Waits for the stream and raises what its kernels flagged: the error word
+// comes with the wait, through a pinned word of the context, so that a call
+// costs one synchronisation (a pageable word took a second one).
+void sync_checked(lima_ctx* c) {
     int* err_ptr = c->p.semantics == LIMA_SEMANTICS_REFERENCE ? c->ref.err : c->phys.err;
-    int h = 0;
-    cuda_ok(cudaMemcpyAsync(&h, err_ptr, sizeof(int), cudaMemcpyDeviceToHost, c->stream), "read error flags");
+    int plain = 0;
+    if (!c->err_word) c->err_word = static_cast<int*>(lima::pinned_alloc(sizeof(int)));
+    int* word = c->err_word ? c->err_word : &plain;
+    *word = 0;
+    cuda_ok(cudaMemcpyAsync(word, err_ptr, sizeof(int), cudaMemcpyDeviceToHost, c->stream), "read error flags");
     cuda_ok(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
+    cuda_ok(cudaGetLastError(), "kernel launch");
+    const int h = *word;
     if (h) {
         cuda_ok(cudaMemsetAsync(err_ptr, 0, sizeof(int), c->stream), "memset");
         cuda_ok(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
@@ -408,12 +418,6 @@ void check_device_errors(lima_ctx* c) {
                               lima::ERR_BIT_PHYS_LIST_OVERFLOW);
         fail(cap ? LIMA_ERR_CAPACITY : LIMA_ERR_NUMERIC, m);
     }
-}
-
-void sync_checked(lima_ctx* c) {
-    cuda_ok(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
-    cuda_ok(cudaGetLastError(), "kernel launch");
-    check_device_errors(c);
 }
 
 void ref_nlist_now(lima_ctx* c) {
@@ -894,26 +898,29 @@ lima_status lima_get_solvents(lima_ctx* c, lima_solvent* sols) {
 lima_status lima_get_positions(lima_ctx* c, float* cxyz, float* sxyz) {
     return guarded(c, [&] {
         need(c->finished, LIMA_ERR_STATE, "lima_finish_box has not run");
-        sync_checked(c);
         const int nc = static_cast<int>(c->comps.size()), ns = static_cast<int>(c->sols.size());
         const size_t ncp = static_cast<size_t>(nc) * lima::kMaxCP;
-        const bool phys = c->p.semantics == LIMA_SEMANTICS_PHYSICS;
+        if (c->p.semantics == LIMA_SEMANTICS_PHYSICS) {
+            // one kernel writes both flat arrays on the device, one copy each into the caller's, one wait
+            if ((!cxyz || nc == 0) && (!sxyz || ns == 0)) {
+                sync_checked(c);
+                return;
+            }
+            const PhysStage g = phys_stage(c);   // the flat arrays take the place of the previous positions and solvents
+            lima_float3* dc = cxyz && nc > 0 ? g.prev : nullptr;
+            lima_float3* ds = sxyz && ns > 0 ? reinterpret_cast<lima_float3*>(g.sols) : nullptr;
+            lima::launch_read_positions(c->phys, c->cur, dc, ds, c->stream);
+            if (dc)
+                cuda_ok(cudaMemcpyAsync(cxyz, dc, sizeof(lima_float3) * ncp, cudaMemcpyDeviceToHost, c->stream), "D2H");
+            if (ds)
+                cuda_ok(cudaMemcpyAsync(sxyz, ds, sizeof(lima_float3) * ns, cudaMemcpyDeviceToHost, c->stream), "D2H");
+            sync_checked(c);
+            return;
+        }
+        sync_checked(c);
         if (cxyz && nc > 0) {
             std::vector<float4> hp(ncp);
-            if (phys) {
-                // the same values lima_get_compound_states gives
-                std::vector<lima_compound_state> st(nc);
-                const PhysStage g = phys_stage(c);
-                lima::launch_read_compounds(c->phys, c->cur, g.states, nullptr, c->stream);
-                cudaMemcpyAsync(st.data(), g.states, sizeof(lima_compound_state) * nc, cudaMemcpyDeviceToHost, c->stream);
-                sync_checked(c);
-                for (size_t k = 0; k < ncp; k++) {
-                    const lima_float3 v = st[k / lima::kMaxCP].positions[k % lima::kMaxCP];
-                    hp[k] = make_float4(v.x, v.y, v.z, 0.f);
-                }
-            } else {
-                cuda_ok(cudaMemcpy(hp.data(), c->ref.cpos[c->cur], sizeof(float4) * ncp, cudaMemcpyDeviceToHost), "D2H");
-            }
+            cuda_ok(cudaMemcpy(hp.data(), c->ref.cpos[c->cur], sizeof(float4) * ncp, cudaMemcpyDeviceToHost), "D2H");
             for (int i = 0; i < nc; i++)
                 for (int t = 0; t < lima::kMaxCP; t++) {
                     const size_t k = static_cast<size_t>(i) * lima::kMaxCP + t;
@@ -924,25 +931,12 @@ lima_status lima_get_positions(lima_ctx* c, float* cxyz, float* sxyz) {
                 }
         }
         if (sxyz && ns > 0) {
-            if (phys) {
-                std::vector<lima_solvent> sv(ns);
-                const PhysStage g = phys_stage(c);
-                lima::launch_read_solvents(c->phys, c->cur, g.sols, c->stream);
-                cudaMemcpyAsync(sv.data(), g.sols, sizeof(lima_solvent) * ns, cudaMemcpyDeviceToHost, c->stream);
-                sync_checked(c);
-                for (int i = 0; i < ns; i++) {
-                    sxyz[3 * i] = sv[i].pos.x;
-                    sxyz[3 * i + 1] = sv[i].pos.y;
-                    sxyz[3 * i + 2] = sv[i].pos.z;
-                }
-            } else {
-                std::vector<float4> a(ns);
-                cuda_ok(cudaMemcpy(a.data(), c->ref.spos[c->cur], sizeof(float4) * ns, cudaMemcpyDeviceToHost), "D2H");
-                for (int i = 0; i < ns; i++) {
-                    sxyz[3 * i] = a[i].x;
-                    sxyz[3 * i + 1] = a[i].y;
-                    sxyz[3 * i + 2] = a[i].z;
-                }
+            std::vector<float4> a(ns);
+            cuda_ok(cudaMemcpy(a.data(), c->ref.spos[c->cur], sizeof(float4) * ns, cudaMemcpyDeviceToHost), "D2H");
+            for (int i = 0; i < ns; i++) {
+                sxyz[3 * i] = a[i].x;
+                sxyz[3 * i + 1] = a[i].y;
+                sxyz[3 * i + 2] = a[i].z;
             }
         }
     });

@@ -1454,6 +1454,38 @@ __global__ void k_read_compounds(PhysDev d, int cur, lima_compound_state* __rest
     if (prev) prev[q] = r;
 }
 
+// positions alone, as flat xyz: compound slots (the values k_read_compounds
+// gives), then solvents
+__global__ void k_read_positions(PhysDev d, int cur, lima_float3* __restrict__ cxyz, lima_float3* __restrict__ sxyz) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x, nc = d.n_c * LIMA_MAX_COMPOUND_PARTICLES;
+    double x[3], v[3];
+    if (q >= nc) {
+        const int s = q - nc;
+        if (s >= d.n_s || !sxyz) return;
+        state_of_orig(d, cur, (uint32_t)(d.n_cp + s), x, v);
+        sxyz[s] = lima_float3{(float)x[0], (float)x[1], (float)x[2]};
+        return;
+    }
+    if (!cxyz) return;
+    const int c = q / LIMA_MAX_COMPOUND_PARTICLES, t = q % LIMA_MAX_COMPOUND_PARTICLES;
+    const uint32_t b = d.cp_base[c];
+    lima_float3 a = {0.f, 0.f, 0.f};
+    if (t < (int)(d.cp_base[c + 1] - b)) {
+        state_of_orig(d, cur, b + t, x, v);
+        if (t > 0) {
+            double x0[3], v0[3];
+            state_of_orig(d, cur, b, x0, v0);
+            const double L = d.L;
+            for (int k = 0; k < 3; k++) {
+                const double dd = x[k] - x0[k];
+                x[k] = x0[k] + (dd - L * nearbyint(dd / L));
+            }
+        }
+        a = lima_float3{(float)x[0], (float)x[1], (float)x[2]};
+    }
+    cxyz[q] = a;
+}
+
 __global__ void k_read_solvents(PhysDev d, int cur, lima_solvent* __restrict__ out) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= d.n_s) return;
@@ -1467,6 +1499,11 @@ __global__ void k_read_solvents(PhysDev d, int cur, lima_solvent* __restrict__ o
 void launch_read_compounds(const PhysDev& d, int cur, lima_compound_state* states, lima_float3* prev, cudaStream_t s) {
     const int n = d.n_c * LIMA_MAX_COMPOUND_PARTICLES;
     if (n > 0) k_read_compounds<<<(n + kTB - 1) / kTB, kTB, 0, s>>>(d, cur, states, prev);
+}
+
+void launch_read_positions(const PhysDev& d, int cur, lima_float3* cxyz, lima_float3* sxyz, cudaStream_t s) {
+    const int n = d.n_c * LIMA_MAX_COMPOUND_PARTICLES + d.n_s;
+    if (n > 0) k_read_positions<<<(n + kTB - 1) / kTB, kTB, 0, s>>>(d, cur, cxyz, sxyz);
 }
 
 void launch_read_solvents(const PhysDev& d, int cur, lima_solvent* out, cudaStream_t s) {

@@ -192,6 +192,8 @@ void phys_energy_now(PhysDev& d, int cur, cudaStream_t s);
 // Either compound output may be null.
 void launch_read_compounds(const PhysDev& d, int cur, lima_compound_state* states, lima_float3* prev, cudaStream_t s);
 void launch_read_solvents(const PhysDev& d, int cur, lima_solvent* out, cudaStream_t s);
+// the same positions as flat xyz (either output may be null)
+void launch_read_positions(const PhysDev& d, int cur, lima_float3* cxyz, lima_float3* sxyz, cudaStream_t s);
 void phys_read_forces(const PhysDev& d, const lima_compound* comps, float4* fc, float4* fs);
 // the Verlet list as CSR over orig ids (offsets[n + 1]; ids, nullable, sorted
 // ascending in each row); returns the total entry count
