@@ -501,7 +501,7 @@ void one_step(lima_ctx* c, cudaEvent_t* prof) {
         } else {   // profiling: the same kernels launched directly, the rebuild decided on the host
             if (dyn_rebuild) {
                 lima::phys_rebuild(c->phys, c->cur, c->stream);
-                c->launches += lima::kRebuildKernels;
+                c->launches += lima::rebuild_kernels(c->phys);
                 c->host_rebuilds++;
             }
             cuda_ok(cudaEventRecord(prof[1], c->stream), "cudaEventRecord");
@@ -514,7 +514,7 @@ void one_step(lima_ctx* c, cudaEvent_t* prof) {
     } else {
         if (rebuild) {
             lima::phys_rebuild(c->phys, c->cur, c->stream);
-            c->launches += lima::kRebuildKernels;
+            c->launches += lima::rebuild_kernels(c->phys);
             c->host_rebuilds++;
             c->last_nlist_step = c->step;
         }
@@ -689,7 +689,7 @@ lima_status lima_finish_box(lima_ctx* c) {
             // grow the capacity to the measured longest row once, and rebuild
             if (lima::phys_fit_list(c->phys, c->stream, c->pool_allocs)) {
                 lima::phys_rebuild(c->phys, c->cur, c->stream);
-                c->launches += lima::kRebuildKernels;
+                c->launches += lima::rebuild_kernels(c->phys);
                 c->host_rebuilds++;
             }
             lima::phys_prime(c->phys, c->cur, c->stream);
@@ -764,7 +764,7 @@ lima_status lima_profile_steps(lima_ctx* c, int n_steps, float* ms) {
         if (c->p.semantics == LIMA_SEMANTICS_PHYSICS && c->phys.dynamic_list &&
             lima::phys_rebuild_pending(c->phys, c->stream)) {
             lima::phys_rebuild(c->phys, c->cur, c->stream);
-            c->launches += lima::kRebuildKernels;
+            c->launches += lima::rebuild_kernels(c->phys);
             c->host_rebuilds++;
         }
         for (int k = 0; k < LIMA_PROF_COUNT; k++) ms[k] = static_cast<float>(acc[k] / n_steps);
@@ -777,7 +777,7 @@ lima_status lima_get_kernel_launches(lima_ctx* c, uint64_t* count) {
         need(count != nullptr, LIMA_ERR_ARGUMENT, "null count");
         *count = c->launches;
         if (c->finished && c->p.semantics == LIMA_SEMANTICS_PHYSICS && c->phys.dynamic_list)
-            *count += lima::phys_device_rebuilds(c->phys, c->stream) * lima::kRebuildKernels;
+            *count += lima::phys_device_rebuilds(c->phys, c->stream) * lima::rebuild_kernels(c->phys);
     });
 }
 
@@ -985,7 +985,7 @@ lima_status lima_set_state(lima_ctx* c, const lima_compound_state* states, const
             lima::phys_upload_state(h, c->phys, c->cur, c->stream);
             lima::phys_rebuild(c->phys, c->cur, c->stream);
             lima::phys_prime(c->phys, c->cur, c->stream);
-            c->launches += lima::kRebuildKernels;
+            c->launches += lima::rebuild_kernels(c->phys);
             c->host_rebuilds++;
             c->last_nlist_step = c->step;
         }
@@ -1020,7 +1020,7 @@ lima_status lima_compute_energies(lima_ctx* c) {
              "the reference computes no LJ energy; reference semantics report potE of the last step");
         if (c->phys.dynamic_list && lima::phys_rebuild_pending(c->phys, c->stream)) {
             lima::phys_rebuild(c->phys, c->cur, c->stream);
-            c->launches += lima::kRebuildKernels;
+            c->launches += lima::rebuild_kernels(c->phys);
             c->host_rebuilds++;
         }
         lima::phys_energy_now(c->phys, c->cur, c->stream);
@@ -1066,7 +1066,7 @@ lima_status lima_build_nlist(lima_ctx* c) {
             ref_nlist_now(c);
         } else {
             lima::phys_rebuild(c->phys, c->cur, c->stream);
-            c->launches += lima::kRebuildKernels;
+            c->launches += lima::rebuild_kernels(c->phys);
             c->host_rebuilds++;
             c->last_nlist_step = c->step;
         }

@@ -11,7 +11,7 @@
 // largely the same neighbours — the position gathers of a warp hit L1.
 //
 // Per step, one launch (captured in a CUDA graph):
-//   k_step   8 lanes per particle walk its Verlet list (blocked so the
+//   k_step   8 or more lanes per particle walk its Verlet list (blocked so the
 //            lanes of consecutive particles read one line), branch-free LJ +
 //            switch; a compound particle's lanes also evaluate the bonded
 //            terms it takes part in and keep its role's force; partial forces
@@ -21,12 +21,12 @@
 //            partials in block order, sets the next step's Berendsen scalar
 //            and, when a particle moved more than skin/2, tail-launches the
 //            rebuild graph, which runs before the next step.
-// Rebuild (a device-launchable graph, or host launches): k_sort_count,
-// k_sort_scan, k_sort_fill, k_sort_order (a stable counting sort by cell),
-// k_permute (every per-slot array into the new order, through tmp arrays)
-// and k_build_list — one warp per 8 particles over the columns of their
-// 5x5x5 cell neighbourhood that their bounding box can reach, which also
-// copies the permuted arrays back.
+// Rebuild (a device-launchable graph, or host launches): k_sort_count (which
+// also scans the counts), k_sort_fill, k_sort_order (a stable counting sort by
+// cell; it also moves every per-slot array into the new order, through tmp
+// arrays) and k_build_list — one warp per one or four particles over the
+// columns of their 5x5x5 cell neighbourhood that their bounding box can
+// reach, which also copies the permuted arrays back.
 #include "physdev.cuh"
 #include "physkern.cuh"
 #include "physmath.cuh"
@@ -66,27 +66,32 @@ __device__ __forceinline__ void cell_xyz(const PhysDev& d, float4 p, int& cx, in
 
 // ----------------------------------------------------- counting sort by cell ---
 // Cell of every slot and its arrival rank in the cell (atomic, so the ranks
-// are put in slot order by k_sort_order).
-__global__ void k_sort_count(PhysDev d, const float4* __restrict__ pos) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= d.n) return;
-    int cx, cy, cz;
-    cell_xyz(d, pos[i], cx, cy, cz);
-    const uint32_t c = (uint32_t)((cx * d.m + cy) * d.m + cz);
-    d.cell_key[i] = c;
-    d.cell_rank[i] = atomicAdd(&d.ccount[c], 1u);
-}
-
-// One block: exclusive scan of the cell occupancies into cstart (cstart[n_cells]
-// = n); the occupancies are reset to zero for the next sort.  Thread t owns a
-// contiguous run of cells.
-__global__ void __launch_bounds__(kScanThreads) k_sort_scan(PhysDev d) {
+// are put in slot order later).  The block that finishes last then scans the
+// cell occupancies into cstart (cstart[n_cells] = n) and resets them to zero
+// for the next sort, thread t owning a contiguous run of cells: a launch of its
+// own for that one block cost about 3 us of a rebuild.
+__global__ void __launch_bounds__(kScanThreads) k_sort_count(PhysDev d, const float4* __restrict__ pos) {
     __shared__ uint32_t s_warp[kScanThreads / 32];
+    __shared__ int s_last;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < d.n) {
+        int cx, cy, cz;
+        cell_xyz(d, pos[i], cx, cy, cz);
+        const uint32_t c = (uint32_t)((cx * d.m + cy) * d.m + cz);
+        d.cell_key[i] = c;
+        d.cell_rank[i] = atomicAdd(&d.ccount[c], 1u);
+    }
+    __threadfence();
+    __syncthreads();
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    if (t == 0) s_last = atomicAdd(d.sort_done, 1u) == gridDim.x - 1u;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
     const int per = (d.n_cells + kScanThreads - 1) / kScanThreads;
-    const int b = t * per, e = min(d.n_cells, b + per);
+    const int b = min(d.n_cells, t * per), e = min(d.n_cells, b + per);
     uint32_t sum = 0u;
-    for (int c = b; c < e; c++) sum += d.ccount[c];
+    for (int c = b; c < e; c++) sum += __ldcg(&d.ccount[c]);
     uint32_t x = sum;   // inclusive scan over the warp
     for (int o = 1; o < 32; o <<= 1) {
         const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
@@ -105,12 +110,15 @@ __global__ void __launch_bounds__(kScanThreads) k_sort_scan(PhysDev d) {
     __syncthreads();
     uint32_t run = (w ? s_warp[w - 1] : 0u) + x - sum;
     for (int c = b; c < e; c++) {
-        const uint32_t k = d.ccount[c];
+        const uint32_t k = __ldcg(&d.ccount[c]);
         d.cstart[c] = run;
         d.ccount[c] = 0u;
         run += k;
     }
-    if (t == 0) d.cstart[d.n_cells] = (uint32_t)d.n;
+    if (t == 0) {
+        d.cstart[d.n_cells] = (uint32_t)d.n;
+        *d.sort_done = 0u;   // for the next sort
+    }
 }
 
 __global__ void k_sort_fill(PhysDev d) {
@@ -119,43 +127,10 @@ __global__ void k_sort_fill(PhysDev d) {
     d.order[d.cstart[d.cell_key[i]] + d.cell_rank[i]] = (uint32_t)i;
 }
 
-// One warp per cell: the cell's slots (in arrival order from k_sort_fill) put
-// in ascending order, which makes the sort stable and the new order a
-// function of the positions and the old order only.  Each lane ranks its slot
-// by counting the smaller ones; cells of more than 32 particles are sorted by
-// lane 0 (insertion sort).
-__global__ void k_sort_order(PhysDev d) {
-    const int lane = threadIdx.x & 31;
-    const int c = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    if (c >= d.n_cells) return;
-    const uint32_t b = d.cstart[c], n = d.cstart[c + 1] - b;
-    if (n <= 1u) return;
-    if (n <= 32u) {
-        const uint32_t v = (uint32_t)lane < n ? d.order[b + lane] : 0xffffffffu;
-        uint32_t rank = 0u;
-        for (uint32_t k = 0; k < n; k++) rank += __shfl_sync(0xffffffffu, v, (int)k) < v ? 1u : 0u;
-        __syncwarp();
-        if ((uint32_t)lane < n) d.order[b + rank] = v;
-        return;
-    }
-    if (lane != 0) return;
-    for (uint32_t k = b + 1; k < b + n; k++) {
-        const uint32_t v = d.order[k];
-        uint32_t j = k;
-        while (j > b && d.order[j - 1] > v) {
-            d.order[j] = d.order[j - 1];
-            j--;
-        }
-        d.order[j] = v;
-    }
-}
-
-// Every per-slot array gathered into cell order (tmp arrays); reference
-// positions of the list; the orig <-> slot maps.
-__global__ void k_permute(PhysDev d, int cur, int mixed) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= d.n) return;
-    const uint32_t src = d.order[k];
+namespace {
+// slot src of the step arrays becomes slot k of the tmp arrays; reference
+// positions of the list; the orig <-> slot maps
+__device__ __forceinline__ void permute_slot(const PhysDev& d, int cur, int mixed, uint32_t src, uint32_t k) {
     const float4 p = d.pos[cur][src];
     d.pos_tmp[0][k] = p;
     d.pos_tmp[1][k] = d.pos[cur ^ 1][src];
@@ -169,6 +144,54 @@ __global__ void k_permute(PhysDev d, int cur, int mixed) {
     d.orig_tmp[k] = o;
     d.sorted_of_orig[o] = k;
     d.xref[k] = p;
+}
+}  // namespace
+
+// One warp per cell: the cell's slots (in arrival order from k_sort_fill) put
+// in ascending order, which makes the sort stable and the new order a
+// function of the positions and the old order only.  Each lane ranks its slot
+// by counting the smaller ones; cells of more than 32 particles are sorted by
+// lane 0 (insertion sort).  PERMUTE: every per-slot array goes into the new
+// order (tmp arrays) here too; else the order goes to d.order.
+template <bool PERMUTE>
+__global__ void k_sort_order(PhysDev d, int cur, int mixed) {
+    const int lane = threadIdx.x & 31;
+    const int c = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (c >= d.n_cells) return;
+    const uint32_t b = d.cstart[c], n = d.cstart[c + 1] - b;
+    if (n == 0u || (!PERMUTE && n == 1u)) return;
+    if (n <= 32u) {
+        const uint32_t v = (uint32_t)lane < n ? d.order[b + lane] : 0xffffffffu;
+        uint32_t rank = 0u;
+        for (uint32_t k = 0; k < n; k++) rank += __shfl_sync(0xffffffffu, v, (int)k) < v ? 1u : 0u;
+        __syncwarp();
+        if ((uint32_t)lane < n) {
+            if (PERMUTE) permute_slot(d, cur, mixed, v, b + rank);
+            else d.order[b + rank] = v;
+        }
+        return;
+    }
+    if (lane == 0)
+        for (uint32_t k = b + 1; k < b + n; k++) {
+            const uint32_t v = d.order[k];
+            uint32_t j = k;
+            while (j > b && d.order[j - 1] > v) {
+                d.order[j] = d.order[j - 1];
+                j--;
+            }
+            d.order[j] = v;
+        }
+    if (PERMUTE) {
+        __threadfence_block();
+        __syncwarp();
+        for (uint32_t k = lane; k < n; k += 32u) permute_slot(d, cur, mixed, d.order[b + k], b + k);
+    }
+}
+
+// every per-slot array into cell order, in large boxes
+__global__ void k_permute(PhysDev d, int cur, int mixed) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < d.n) permute_slot(d, cur, mixed, d.order[k], (uint32_t)k);
 }
 
 __global__ void k_set_xref(PhysDev d, const float4* __restrict__ pos) {
@@ -403,7 +426,7 @@ __device__ __forceinline__ void scan_stream(const PhysDev& d, const float4* __re
 }  // namespace
 
 template <typename ID, int P>
-__global__ void __launch_bounds__(kBuildWarps * 32, P == 1 ? 8 : 6) k_build_list(const __grid_constant__ PhysDev d,
+__global__ void __launch_bounds__(kBuildWarps * 32, P == 1 ? 8 : 0) k_build_list(const __grid_constant__ PhysDev d,
                                                                  const float4* __restrict__ pos,
                                                                  const uint32_t* __restrict__ orig,
                                                                  const uint32_t* __restrict__ items, int copy_cur,
@@ -1304,6 +1327,9 @@ namespace {
 // The step kernel with a programmatic dependency on the kernel before it in
 // the stream (the bonded kernel): it may start before that one has finished
 // and waits for it only where it reads its results.
+bool has_bonded(const PhysDev& d) { return d.n_bonds + d.n_angles + d.n_dih > 0; }
+
+// (without bonded terms no bonded kernel comes before it: an ordinary launch)
 template <typename K>
 void launch_programmatic(K kernel, const PhysDev& d, int blocks, int cur, int slot, cudaGraphExec_t tail, size_t smem,
                          cudaStream_t s) {
@@ -1316,7 +1342,7 @@ void launch_programmatic(K kernel, const PhysDev& d, int blocks, int cur, int sl
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = has_bonded(d) ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kernel, d, cur, slot, tail);
 }
 
@@ -1363,15 +1389,27 @@ void step_tail(const PhysDev& d, int cur, int slot, cudaGraphExec_t tail, cudaSt
 
 }  // namespace
 
-void launch_sort(const PhysDev& d, const float4* pos, cudaStream_t s) {
-    k_sort_count<<<(d.n + kTB - 1) / kTB, kTB, 0, s>>>(d, pos);
-    k_sort_scan<<<1, kScanThreads, 0, s>>>(d);
+namespace {
+void sort_cells(const PhysDev& d, const float4* pos, cudaStream_t s) {
+    k_sort_count<<<(d.n + kScanThreads - 1) / kScanThreads, kScanThreads, 0, s>>>(d, pos);
     k_sort_fill<<<(d.n + kTB - 1) / kTB, kTB, 0, s>>>(d);
-    k_sort_order<<<(int)(((size_t)d.n_cells * 32 + kTB - 1) / kTB), kTB, 0, s>>>(d);
+}
+int order_blocks(const PhysDev& d) { return (int)(((size_t)d.n_cells * 32 + kTB - 1) / kTB); }
+}  // namespace
+
+void launch_sort(const PhysDev& d, const float4* pos, cudaStream_t s) {
+    sort_cells(d, pos, s);
+    k_sort_order<false><<<order_blocks(d), kTB, 0, s>>>(d, 0, 0);
 }
 
-void launch_permute(const PhysDev& d, int cur, bool mixed, cudaStream_t s) {
-    k_permute<<<(d.n + kTB - 1) / kTB, kTB, 0, s>>>(d, cur, mixed ? 1 : 0);
+void launch_sort_permute(const PhysDev& d, int cur, bool mixed, cudaStream_t s) {
+    sort_cells(d, d.pos[cur], s);
+    if (d.n < kPermuteAloneFrom) {
+        k_sort_order<true><<<order_blocks(d), kTB, 0, s>>>(d, cur, mixed ? 1 : 0);
+    } else {
+        k_sort_order<false><<<order_blocks(d), kTB, 0, s>>>(d, cur, 0);
+        k_permute<<<(d.n + kTB - 1) / kTB, kTB, 0, s>>>(d, cur, mixed ? 1 : 0);
+    }
 }
 
 void launch_set_xref(const PhysDev& d, const float4* pos, cudaStream_t s) {
@@ -1510,8 +1548,9 @@ void launch_read_solvents(const PhysDev& d, int cur, lima_solvent* out, cudaStre
     if (d.n_s > 0) k_read_solvents<<<(d.n_s + kTB - 1) / kTB, kTB, 0, s>>>(d, cur, out);
 }
 
-void launch_bonded(const PhysDev& d, int cur, bool energy, cudaStream_t s) {
+int launch_bonded(const PhysDev& d, int cur, bool energy, cudaStream_t s) {
     const int nb = bonded_blocks(d);
+    if (nb == 0) return 0;
     const bool mixed = d.precision == LIMA_PRECISION_MIXED;
     if (energy && mixed)
         k_bonded<true, true><<<nb, kTB, 0, s>>>(d, cur);
@@ -1521,6 +1560,7 @@ void launch_bonded(const PhysDev& d, int cur, bool energy, cudaStream_t s) {
         k_bonded<false, true><<<nb, kTB, 0, s>>>(d, cur);
     else
         k_bonded<false, false><<<nb, kTB, 0, s>>>(d, cur);
+    return 1;
 }
 
 void launch_step(const PhysDev& d, int cur, bool mixed, bool energy, bool integrate, int slot, cudaGraphExec_t tail,

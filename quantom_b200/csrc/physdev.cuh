@@ -87,6 +87,7 @@ struct PhysDev {
     uint32_t* cell_rank;        // [n] arrival order of the slot in its cell
     uint32_t* ccount;           // [n_cells] occupancy during a sort; zero between sorts
     uint32_t* order;            // [n] slots in cell order
+    unsigned int* sort_done;    // blocks of the count that have finished; zero between sorts
     uint32_t* cstart;           // [n_cells + 1]: cell c holds sorted slots [cstart[c], cstart[c+1])
     float4* pos_tmp[2]; float4* vel_tmp; float4* posc_tmp; float4* velc_tmp; float4* force_tmp; uint32_t* orig_tmp;
     // Verlet list (tile-local indices)
@@ -172,8 +173,13 @@ unsigned long long phys_device_rebuilds(const PhysDev& d, cudaStream_t s);
 // the device-launchable rebuild graphs of both parities (after the list capacity is final)
 int phys_capture_rebuild(PhysDev& d, cudaStream_t s, std::string& msg);
 void phys_free_rebuild(PhysDev& d);
-// k_sort_count, k_sort_scan, k_sort_fill, k_sort_order, k_permute, k_build_list
-constexpr int kRebuildKernels = 6;
+// From this box size on the rebuild moves the per-slot arrays in a kernel of its
+// own, a thread per slot; below, the warp that orders a cell moves its slots
+// too (about a third of its lanes have one: 32,024 particles a host-issued
+// rebuild 106 -> 103 us with the launch it saves, 258,192 565 -> 592).
+constexpr int kPermuteAloneFrom = 131072;
+// k_sort_count, k_sort_fill, k_sort_order, (k_permute), k_build_list
+inline int rebuild_kernels(const PhysDev& d) { return d.n < kPermuteAloneFrom ? 4 : 5; }
 // One step: the bonded kernel, then the step kernel (pair terms,
 // integration, FP64 sums) launched programmatically so that it overlaps the
 // bonded kernel.  tail: launch the due rebuild from the device (the launch

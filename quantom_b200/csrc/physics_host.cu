@@ -349,6 +349,7 @@ int phys_setup(const PhysHost& h, PhysDev& d, cudaStream_t s, std::vector<void*>
         d.part = a.take<double>((size_t)std::max(step_blocks(d, false), step_blocks(d, true)) * kRedStride);
         d.bpart = a.take<double>((size_t)bonded_blocks(d) * 4);
         d.done = a.take<unsigned int>(1);
+        d.sort_done = a.take<unsigned int>(1);
         d.e_last = a.take<double>(LIMA_E_COUNT);
         d.lambda = a.take<float>(2);
         d.err = a.take<int>(1);
@@ -390,6 +391,7 @@ int phys_setup(const PhysHost& h, PhysDev& d, cudaStream_t s, std::vector<void*>
     }
     cudaMemsetAsync(d.ccount, 0, sizeof(uint32_t) * d.n_cells, s);
     cudaMemsetAsync(d.done, 0, sizeof(unsigned int), s);
+    cudaMemsetAsync(d.sort_done, 0, sizeof(unsigned int), s);
     cudaMemsetAsync(d.e_last, 0, sizeof(double) * LIMA_E_COUNT, s);
     cudaMemsetAsync(d.err, 0, sizeof(int), s);
     cudaMemsetAsync(d.need_rebuild, 0, sizeof(int), s);
@@ -485,8 +487,7 @@ void phys_upload_state(const PhysHost& h, PhysDev& d, int cur, cudaStream_t s) {
 
 void phys_rebuild(const PhysDev& d, int cur, cudaStream_t s) {
     const bool mixed = d.precision == LIMA_PRECISION_MIXED;
-    launch_sort(d, d.pos[cur], s);
-    launch_permute(d, cur, mixed, s);
+    launch_sort_permute(d, cur, mixed, s);
     launch_build_list(d, d.pos_tmp[0], d.orig_tmp, nullptr, cur, mixed, s);
 }
 
@@ -618,12 +619,12 @@ int phys_capture_dynamic(const PhysDev& d, int cur, bool energy, cudaStream_t s,
 // with lambda[cur] and sets lambda[cur ^ 1] from its kinetic energy.
 int phys_step_kernels(const PhysDev& d, int cur, cudaStream_t s, bool energy, cudaEvent_t* ev, bool tail) {
     if (ev) cudaEventRecord(ev[0], s);
-    launch_bonded(d, cur, energy, s);
+    const int bonded = launch_bonded(d, cur, energy, s);
     if (ev) cudaEventRecord(ev[1], s);
     launch_step(d, cur, d.precision == LIMA_PRECISION_MIXED, energy, true, cur, tail ? d.rebuild_exec[cur ^ 1] : nullptr,
                 s);
     if (ev) cudaEventRecord(ev[2], s);
-    return 2;
+    return 1 + bonded;
 }
 
 void phys_energy_now(PhysDev& d, int cur, cudaStream_t s) {

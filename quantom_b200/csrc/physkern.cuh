@@ -69,16 +69,16 @@ __host__ __device__ inline size_t nl_entry_bytes(const PhysDev& d) { return d.nl
 // lanes that walk one particle's list in the step kernel, and its blocks
 int step_lanes(const PhysDev& d, bool energy);
 int step_blocks(const PhysDev& d, bool energy);
-// blocks of the bonded kernel (one thread per term)
+// blocks of the bonded kernel (one thread per term; none without terms)
 __host__ __device__ inline int bonded_blocks(const PhysDev& d) {
     const int nt = d.n_bonds + d.n_angles + d.n_dih;
-    return nt > 0 ? (nt + kTB - 1) / kTB : 1;
+    return (nt + kTB - 1) / kTB;
 }
 
 // the counting sort of the slots by the cell of `pos`: cell_key, cstart, order
 void launch_sort(const PhysDev& d, const float4* pos, cudaStream_t s);
-// every per-slot array into cell order in the tmp arrays, reference positions
-void launch_permute(const PhysDev& d, int cur, bool mixed, cudaStream_t s);
+// the sort by the cell of pos[cur], and every per-slot array into cell order in the tmp arrays, reference positions
+void launch_sort_permute(const PhysDev& d, int cur, bool mixed, cudaStream_t s);
 // reference positions of an in-place build (particles not moved)
 void launch_set_xref(const PhysDev& d, const float4* pos, cudaStream_t s);
 // The Verlet list of positions pos (orig: orig ids by slot).  items
@@ -87,8 +87,8 @@ void launch_set_xref(const PhysDev& d, const float4* pos, cudaStream_t s);
 // every tmp array back into the step arrays of that parity.
 void launch_build_list(const PhysDev& d, const float4* pos, const uint32_t* orig, const uint32_t* items, int copy_cur,
                        bool mixed, cudaStream_t s);
-// The bonded kernel of parity `cur` (term forces; ENERGY: block partials)
-void launch_bonded(const PhysDev& d, int cur, bool energy, cudaStream_t s);
+// The bonded kernel of parity `cur` (term forces; ENERGY: block partials); returns the kernels launched
+int launch_bonded(const PhysDev& d, int cur, bool energy, cudaStream_t s);
 // The step kernel of parity `cur` (slot cur) or an energy evaluation (slot
 // kSlotEval, integrate false), launched with a programmatic dependency on the
 // bonded kernel before it.  tail: device-launchable rebuild graph the last
