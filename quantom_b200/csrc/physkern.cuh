@@ -8,7 +8,7 @@
 namespace lima {
 
 constexpr int kTB = 256;         // threads per block of the per-particle kernels and the step kernel
-constexpr int kGroup = 8;        // lanes per particle in the list and step kernels
+constexpr int kGroup = 8;        // columns of the list: the lanes of a particle come in groups of 8
 constexpr int kBuildWarps = 4;   // warps per block of the list build
 // The list build gives a warp one particle below this box size (more warps,
 // shorter streams) and four from it on (fewer tests and one stream's fetches
