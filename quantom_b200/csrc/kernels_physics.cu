@@ -346,10 +346,13 @@ __device__ __forceinline__ void flush_rows(const PhysDev& d, const uint32_t* __r
     }
 }
 
-// The group's candidate stream (`total` of them, at least one; n_ranges ranges
-// in rg, their first stream indices in rstart) against its particles: px..
-// (NaN: not in the group) at cell-order positions first, first + 1, ...
-// ITEMS: the cell order is a list of slots.
+// The group's candidate stream (`total` of them, the same in every lane;
+// n_ranges ranges in rg, their first stream indices in rstart) against its
+// particles: px.. (NaN: not in the group) at cell-order positions first,
+// first + 1, ...  ITEMS: the cell order is a list of slots.
+// A stream can be empty: a particle that is alone in its group and not finite,
+// or more than the list radius outside the box, reaches none of the columns
+// around its clamped cell.  It then has no range to fetch from.
 template <bool MIN_IMAGE, bool ITEMS, typename ID, int P>
 __device__ __forceinline__ void scan_stream(const PhysDev& d, const float4* __restrict__ pos,
                                             const uint32_t* __restrict__ items, const BuildRange* rg, const int* rstart,
@@ -357,6 +360,7 @@ __device__ __forceinline__ void scan_stream(const PhysDev& d, const float4* __re
                                             ID* rows, int i, uint32_t (&done)[P], const float (&px)[P],
                                             const float (&py)[P], const float (&pz)[P], uint32_t row, uint32_t cap,
                                             uint32_t (&cnt)[P], int lane) {
+    if (total <= 0) return;
     constexpr uint32_t kB = sizeof(ID);
     const uint32_t lt = (1u << lane) - 1u, le = lt | (1u << lane);
     const float rl2 = d.rlist2, nan = __int_as_float(0x7fc00000), L = d.L, invL = d.invL;

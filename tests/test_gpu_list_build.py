@@ -67,3 +67,33 @@ def test_list_is_the_brute_force_list(box, waters, chains, length, cutoff):
         want = (want[:, 0] + lo) * n + want[:, 1]
         want = want[~torch.isin(want, ex)]
         assert torch.isin(want, mine).all()
+
+
+@pytest.mark.parametrize("box,waters", [(4.0, 1901), (8.1, 16385)])   # one and four particles a warp
+@pytest.mark.parametrize("axis,value", [(0, np.nan), (1, np.nan), (2, np.nan), (0, np.inf)])
+def test_particle_without_candidates(box, waters, axis, value):
+    """A particle that is not finite on some axis has an empty candidate stream:
+    its row is empty, the others' rows are those of the box without it, the next
+    step reports it, and the engine goes on from a finite state."""
+    spec = S.SystemSpec("box", box, waters, cutoff=1.0, mc_sweeps=4)
+    s = S.make_system(spec, seed=12)
+    p = E.default_params(box_len=box, cutoff=1.0, dt=spec.dt, semantics=E.SEMANTICS_PHYSICS, skin=0.05, switch_on=0.8,
+                         nlist_period=0)
+    lost = waters // 3
+    bad = s.solvents.copy()
+    bad["pos"][lost, axis] = value
+    with E.Engine(s, p) as eng:
+        off, ids = (np.asarray(a).copy() for a in eng.nlist(E.NL_PAIR))
+        rows = np.repeat(np.arange(waters), np.diff(off))
+        eng.set_state(s.states, None, bad)
+        boff, bids = eng.nlist(E.NL_PAIR)
+        brows = np.repeat(np.arange(waters), np.diff(boff))
+        keep = (rows != lost) & (ids != lost)
+        assert np.array_equal(brows, rows[keep]) and np.array_equal(bids, ids[keep])
+        with pytest.raises(E.LimaError) as ei:
+            eng.step(1)
+            eng.synchronize()
+        assert ei.value.status == E.ERR_NUMERIC
+        eng.set_state(s.states, None, s.solvents)
+        goff, gids = eng.nlist(E.NL_PAIR)
+        assert np.array_equal(goff, off) and np.array_equal(gids, ids)
