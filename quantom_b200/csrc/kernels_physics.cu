@@ -27,6 +27,7 @@
 // arrays) and k_build_list — one warp per one or four particles over the
 // columns of their 5x5x5 cell neighbourhood that their bounding box can
 // reach, which also copies the permuted arrays back.
+#include "cellrange.cuh"
 #include "physdev.cuh"
 #include "physkern.cuh"
 #include "physmath.cuh"
@@ -57,9 +58,9 @@ __device__ __forceinline__ double warp_sum(double v) {
 
 __device__ __forceinline__ void cell_xyz(const PhysDev& d, float4 p, int& cx, int& cy, int& cz) {
     const float inv = (float)d.m / d.L;
-    cx = min(max((int)(p.x * inv), 0), d.m - 1);
-    cy = min(max((int)(p.y * inv), 0), d.m - 1);
-    cz = min(max((int)(p.z * inv), 0), d.m - 1);
+    cx = cell_of(p.x, inv, d.m);
+    cy = cell_of(p.y, inv, d.m);
+    cz = cell_of(p.z, inv, d.m);
 }
 
 }  // namespace
@@ -506,55 +507,34 @@ __global__ void __launch_bounds__(kBuildWarps * 32, P == 1 ? 8 : 0) k_build_list
             todo &= ~__reduce_or_sync(0xffffffffu, mine ? 1u << lane : 0u);
             const int hz1 = __reduce_max_sync(0xffffffffu, mine ? cz : -1);   // the group's top cell
             members(mine);
-            float bxl = 3.4e38f, bxh = -3.4e38f, byl = 3.4e38f, byh = -3.4e38f, bzl = 3.4e38f, bzh = -3.4e38f;
+            GroupBox b = {3.4e38f, -3.4e38f, 3.4e38f, -3.4e38f, 3.4e38f, -3.4e38f};
 #pragma unroll
             for (int p = 0; p < P; p++) {   // a NaN x marks a particle outside the group
                 const bool in = px[p] == px[p];
-                bxl = fminf(bxl, px[p]);
-                bxh = fmaxf(bxh, px[p]);
-                byl = in ? fminf(byl, py[p]) : byl;
-                byh = in ? fmaxf(byh, py[p]) : byh;
-                bzl = in ? fminf(bzl, pz[p]) : bzl;
-                bzh = in ? fmaxf(bzh, pz[p]) : bzh;
+                b.xl = fminf(b.xl, px[p]);
+                b.xh = fmaxf(b.xh, px[p]);
+                b.yl = in ? fminf(b.yl, py[p]) : b.yl;
+                b.yh = in ? fmaxf(b.yh, py[p]) : b.yh;
+                b.zl = in ? fminf(b.zl, pz[p]) : b.zl;
+                b.zh = in ? fmaxf(b.zh, pz[p]) : b.zh;
             }
-            // lane c < 25: column (hx + c / 5 - 2, hy + c % 5 - 2), one or two ranges
+            // lane c < 25: column (hx + c / 5 - 2, hy + c % 5 - 2), one or two ranges of slots
             int b0 = 0, l0 = 0, b1 = 0, l1 = 0;
             float sx = 0.f, sy = 0.f, sz0 = 0.f, sz1 = 0.f;
             if (lane < 25) {
-                const int ox = lane / 5 - 2, oy = lane % 5 - 2;
-                const float cxl = (float)(hx + ox) * cs, cxh = cxl + cs;   // unwrapped, home frame
-                const float cyl = (float)(hy + oy) * cs, cyh = cyl + cs;
-                const float gx = fmaxf(0.f, fmaxf(cxl - bxh, bxl - cxh));
-                const float gy = fmaxf(0.f, fmaxf(cyl - byh, byl - cyh));
-                const float g2 = gx * gx + gy * gy;
-                if (g2 < d.rlist2 * 1.0001f) {   // the margin covers cell rounding
-                    int x = hx + ox, y = hy + oy;
-                    if (x < 0) { x += m; sx = -d.L; } else if (x >= m) { x -= m; sx = d.L; }
-                    if (y < 0) { y += m; sy = -d.L; } else if (y >= m) { y -= m; sy = d.L; }
-                    const int col = (x * m + y) * m;
-                    // cells within the reach of the group's z-range (unwrapped; at
-                    // most m of them: the group spans <= m - 4 cells).  Both ends
-                    // clamped: a position far outside the box stays inside cstart.
-                    const float reach = sqrtf(fmaxf(d.rlist2 - g2, 0.f)) + 1e-4f * cs;
-                    const int u0 = min(max((int)floorf((bzl - reach) * ics), hz0 - 2), hz1 + 2);
-                    const int u1 = max(min((int)floorf((bzh + reach) * ics), hz1 + 2), u0 - 1);
-                    if (u0 < 0) {
-                        b0 = (int)d.cstart[col + u0 + m];
-                        l0 = (int)d.cstart[col + m] - b0;
-                        sz0 = -d.L;
-                        b1 = (int)d.cstart[col];
-                        l1 = (int)d.cstart[col + u1 + 1] - b1;
-                    } else if (u1 >= m) {
-                        b0 = (int)d.cstart[col + u0];
-                        l0 = (int)d.cstart[col + m] - b0;
-                        b1 = (int)d.cstart[col];
-                        l1 = (int)d.cstart[col + u1 - m + 1] - b1;
-                        sz1 = d.L;
-                    } else if (u1 >= u0) {
-                        b0 = (int)d.cstart[col + u0];
-                        l0 = (int)d.cstart[col + u1 + 1] - b0;
-                    }
+                const ColumnCells o = column_cells(lane, m, d.L, cs, ics, d.rlist2, hx, hy, hz0, hz1, b);
+                if (o.n0 > 0) {
+                    b0 = (int)d.cstart[o.c0];
+                    l0 = (int)d.cstart[o.c0 + o.n0] - b0;
                 }
+                if (o.n1 > 0) {
+                    b1 = (int)d.cstart[o.c1];
+                    l1 = (int)d.cstart[o.c1 + o.n1] - b1;
+                }
+                sx = o.sx;
+                sy = o.sy;
+                sz0 = o.sz0;
+                sz1 = o.sz1;
             }
             // stream offsets: inclusive scan of the per-column lengths; the non-empty ranges in column order
             const int len = l0 + l1;
@@ -564,7 +544,7 @@ __global__ void __launch_bounds__(kBuildWarps * 32, P == 1 ? 8 : 0) k_build_list
                 const int y = __shfl_up_sync(0xffffffffu, incl, o);
                 if (lane >= o) incl += y;
             }
-            const int total = uniform(incl);
+            const int total = uniform(incl);   // the last lane's: no length is negative
             const unsigned has0 = __ballot_sync(0xffffffffu, l0 > 0), has1 = __ballot_sync(0xffffffffu, l1 > 0);
             const unsigned lt = (1u << lane) - 1u;
             int at = __popc(has0 & lt) + __popc(has1 & lt);

@@ -97,3 +97,32 @@ def test_particle_without_candidates(box, waters, axis, value):
         eng.set_state(s.states, None, s.solvents)
         goff, gids = eng.nlist(E.NL_PAIR)
         assert np.array_equal(goff, off) and np.array_equal(gids, ids)
+
+
+@pytest.mark.parametrize("apart", [0.001, 0.02, 0.04, 0.06, 0.08, 0.1])
+@pytest.mark.parametrize("axis", [0, 2])
+def test_rebuild_with_particles_thrown_out_of_the_box(apart, axis):
+    """Two waters too close together are thrown up to many box lengths away (or
+    to infinity) within a step, which asks for a rebuild at those positions: a
+    numeric status or none, and the engine goes on from an ordinary state."""
+    box, waters = 4.0, 1900
+    spec = S.SystemSpec("box", box, waters, cutoff=1.0, mc_sweeps=4)
+    s = S.make_system(spec, seed=13)
+    p = E.default_params(box_len=box, cutoff=1.0, dt=spec.dt, semantics=E.SEMANTICS_PHYSICS, skin=0.05, switch_on=0.8,
+                         nlist_period=0)
+    close = s.solvents.copy()
+    close["pos"][1] = close["pos"][0]
+    close["pos"][1, axis] += np.float32(apart)
+    close["pos_tsub1"][:2] = close["pos"][:2]
+    with E.Engine(s, p) as eng:
+        off, ids = (np.asarray(a).copy() for a in eng.nlist(E.NL_PAIR))
+        eng.set_state(s.states, None, close)
+        try:
+            for _ in range(6):
+                eng.step(1)
+                eng.synchronize()
+        except E.LimaError as e:
+            assert e.status == E.ERR_NUMERIC
+        eng.set_state(s.states, None, s.solvents)
+        goff, gids = eng.nlist(E.NL_PAIR)
+        assert np.array_equal(goff, off) and np.array_equal(gids, ids)
