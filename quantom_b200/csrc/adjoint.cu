@@ -148,6 +148,9 @@ struct AdjArgs {
 // weights per bin; the block's lanes are summed in FP64.  8,192 particles, 50
 // bins on one B200: shared-memory 64-bit atomics, three per pair, took 87 us.
 constexpr int kLossTB = 128;
+// its static shared memory (warp energies and the LJ table), which counts
+// towards the 48 KB that a launch gets without asking
+constexpr size_t kLossStaticSmem = sizeof(double) * (kLossTB / 32) + sizeof(float2) * kMaxTypes * kMaxTypes;
 template <typename ID>
 __global__ void __launch_bounds__(kLossTB) k_loss_pairs(PhysDev d, const float4* __restrict__ pos, int n_bins,
                                                         float inv_dr, float supp2, double inv_n,
@@ -394,6 +397,7 @@ __global__ void k_adj_prep(PhysDev d, AdjArgs a, float4* __restrict__ lam_v, flo
 // 8,192 particles on one B200: 55 us with per-thread arrays indexed by type
 // (local memory) and four IEEE divisions an entry.
 constexpr int kAdjPairTB = 128;
+constexpr size_t kAdjPairStaticSmem = sizeof(float) * (LIMA_LOSS_MAX_BINS + 8);
 template <bool HVP, bool LOSS, typename ID, int LANES>
 __global__ void __launch_bounds__(kAdjPairTB) k_adj_pair(PhysDev d, const float4* __restrict__ pos, AdjArgs a,
                                                          const double* __restrict__ hist_n,
@@ -785,7 +789,8 @@ struct Runner {
     void loss_pass(int cur, const float4* pos, const float4* po, int n) {
         const size_t smem = sizeof(float) * 32 * (kLossTB / 32) * (n_bins + 4);
         auto run = [&](auto kernel) {
-            if (smem > 40 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (smem + kLossStaticSmem > kSmemPlain)
+                cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             kernel<<<blocks_pair(kLossTB, kGroup), kLossTB, smem, s>>>(d, pos, n_bins, inv_dr, supp2, 1.0 / d.n, A.U + n,
                                                                A.hist + (size_t)n * n_bins);
         };
@@ -804,7 +809,8 @@ struct Runner {
         const size_t smem = sizeof(float4) * nt2 + sizeof(float2) * (nt2 + (nt2 & 1)) +
                             sizeof(float) * 32 * (kAdjPairTB / 32) * 2 * a.n_types;
         auto run = [&](auto kernel) {
-            if (smem > 40 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (smem + kAdjPairStaticSmem > kSmemPlain)
+                cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             kernel<<<blocks_pair(kAdjPairTB, pair_lanes(d.n)), kAdjPairTB, smem, s>>>(d, xs, a, hist_n, A.target);
         };
         if (pair_lanes(d.n) == 16) {

@@ -18,6 +18,9 @@ constexpr int kBuildWarps = 4;   // warps per block of the list build
 constexpr int kBuildOneBelow = 16384;
 constexpr int kMaxTypes = 32;    // LIMA_MAX_ATOM_TYPES
 constexpr int kScanThreads = 1024;
+// shared memory, static and dynamic together, that a block gets without the
+// kernel's MaxDynamicSharedMemorySize being raised
+constexpr size_t kSmemPlain = 48 * 1024;
 
 // Lanes per particle in the step kernel: 8 (one list column each), more in
 // boxes too small to fill the SMs' warps, where a lane's chain of chunk loads

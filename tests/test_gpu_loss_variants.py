@@ -57,3 +57,21 @@ def test_gradient_matches_fp64_differences(box, waters, chains):
         e[k] = 1e-4 * abs(th[k])
         fd = (value(th + e) - value(th - e)) / (2 * e[k])
         assert abs(g[k] - fd) < 1e-3 * abs(fd), (k, g[k], fd)
+
+
+@pytest.mark.parametrize("bins", [75, 76, 77])
+def test_bins_around_the_plain_shared_memory_limit(bins, tmp_path):
+    """The loss kernel's columns of 76 bins and its static arrays together pass
+    the 48 KB a launch gets unasked.  Each count in a process of its own: a
+    larger count would raise the kernel's limit for those after it."""
+    import subprocess
+    import sys
+    from conftest import ROOT
+    code = ("from quantom_b200 import engine as E, systems as S\n"
+            "s = S.make_system('tiny_solvent', seed=3)\n"
+            "p = E.default_params(box_len=s.spec.box_len, cutoff=s.spec.cutoff, dt=s.spec.dt, "
+            "semantics=E.SEMANTICS_PHYSICS, skin=0.1, switch_on=1.0, nlist_period=0)\n"
+            f"h = E.Engine(s, p).rdf({bins}, 1.0)\n"
+            "assert h.sum() > 0\n")
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
