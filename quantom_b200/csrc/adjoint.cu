@@ -151,6 +151,7 @@ constexpr int kLossTB = 128;
 // its static shared memory (warp energies and the LJ table), which counts
 // towards the 48 KB that a launch gets without asking
 constexpr size_t kLossStaticSmem = sizeof(double) * (kLossTB / 32) + sizeof(float2) * kMaxTypes * kMaxTypes;
+constexpr size_t loss_smem(int n_bins) { return sizeof(float) * 32 * (kLossTB / 32) * (n_bins + 4); }
 template <typename ID>
 __global__ void __launch_bounds__(kLossTB) k_loss_pairs(PhysDev d, const float4* __restrict__ pos, int n_bins,
                                                         float inv_dr, float supp2, double inv_n,
@@ -398,6 +399,10 @@ __global__ void k_adj_prep(PhysDev d, AdjArgs a, float4* __restrict__ lam_v, flo
 // (local memory) and four IEEE divisions an entry.
 constexpr int kAdjPairTB = 128;
 constexpr size_t kAdjPairStaticSmem = sizeof(float) * (LIMA_LOSS_MAX_BINS + 8);
+constexpr size_t adj_pair_smem(int nt) {
+    return sizeof(float4) * nt * nt + sizeof(float2) * (nt * nt + (nt * nt & 1)) +
+           sizeof(float) * 32 * (kAdjPairTB / 32) * 2 * nt;
+}
 template <bool HVP, bool LOSS, typename ID, int LANES>
 __global__ void __launch_bounds__(kAdjPairTB) k_adj_pair(PhysDev d, const float4* __restrict__ pos, AdjArgs a,
                                                          const double* __restrict__ hist_n,
@@ -787,10 +792,9 @@ struct Runner {
     }
     // energy and occupancies of the state in parity cur -> U[n], hist[n]
     void loss_pass(int cur, const float4* pos, const float4* po, int n) {
-        const size_t smem = sizeof(float) * 32 * (kLossTB / 32) * (n_bins + 4);
+        const size_t smem = loss_smem(n_bins);
         auto run = [&](auto kernel) {
-            if (smem + kLossStaticSmem > kSmemPlain)
-                cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            allow_smem(kernel, smem, kLossStaticSmem, loss_smem(LIMA_LOSS_MAX_BINS));
             kernel<<<blocks_pair(kLossTB, kGroup), kLossTB, smem, s>>>(d, pos, n_bins, inv_dr, supp2, 1.0 / d.n, A.U + n,
                                                                A.hist + (size_t)n * n_bins);
         };
@@ -805,12 +809,9 @@ struct Runner {
     // one adjoint pair pass over the state xs (hist_n: its occupancies, with a loss term)
     template <bool HVP, bool LOSS>
     void adj_pair(const float4* xs, const AdjArgs& a, const double* hist_n) {
-        const int nt2 = a.n_types * a.n_types;
-        const size_t smem = sizeof(float4) * nt2 + sizeof(float2) * (nt2 + (nt2 & 1)) +
-                            sizeof(float) * 32 * (kAdjPairTB / 32) * 2 * a.n_types;
+        const size_t smem = adj_pair_smem(a.n_types);
         auto run = [&](auto kernel) {
-            if (smem + kAdjPairStaticSmem > kSmemPlain)
-                cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            allow_smem(kernel, smem, kAdjPairStaticSmem, adj_pair_smem(kMaxTypes));
             kernel<<<blocks_pair(kAdjPairTB, pair_lanes(d.n)), kAdjPairTB, smem, s>>>(d, xs, a, hist_n, A.target);
         };
         if (pair_lanes(d.n) == 16) {

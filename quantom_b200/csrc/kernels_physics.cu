@@ -1409,8 +1409,7 @@ void build_list(const PhysDev& d, const float4* pos, const uint32_t* orig, const
     const int warps = (d.n + P - 1) / P;
     const int cap = std::min(d.nl_cap, kBuildRow);
     const size_t smem = kBuildWarps * build_warp_smem(P, cap, sizeof(ID));
-    if (smem > kSmemPlain)
-        cudaFuncSetAttribute(k_build_list<ID, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(k_build_list<ID, P>, smem, 0, kBuildWarps * build_warp_smem(P, kBuildRow, sizeof(ID)));
     k_build_list<ID, P><<<(warps + kBuildWarps - 1) / kBuildWarps, kBuildWarps * 32, smem, s>>>(
         d, pos, orig, items, copy_cur, mixed ? 1 : 0, cap);
 }

@@ -21,6 +21,17 @@ constexpr int kScanThreads = 1024;
 // shared memory, static and dynamic together, that a block gets without the
 // kernel's MaxDynamicSharedMemorySize being raised
 constexpr size_t kSmemPlain = 48 * 1024;
+// Before a launch with `dynamic` bytes of a kernel that has `fixed` static
+// ones.  The limit belongs to the kernel and is shared by every context and
+// host thread of the process, so it is only ever set to `most`, the largest
+// size the kernel is launched with: set to each launch's own size, one thread
+// could lower it between another's call here and its launch.  A failure is the
+// error that cudaGetLastError gives next.
+template <typename K>
+inline void allow_smem(K kernel, size_t dynamic, size_t fixed, size_t most) {
+    if (dynamic + fixed > kSmemPlain)
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
 
 // Lanes per particle in the step kernel: 8 (one list column each), more in
 // boxes too small to fill the SMs' warps, where a lane's chain of chunk loads

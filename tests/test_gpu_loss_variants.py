@@ -75,3 +75,29 @@ def test_bins_around_the_plain_shared_memory_limit(bins, tmp_path):
             "assert h.sum() > 0\n")
     r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+def test_threads_with_different_bins():
+    """Engines on eight host threads whose loss kernels need two different amounts
+    of shared memory beyond the plain limit: no launch is refused."""
+    import threading
+    s = S.make_system("tiny_solvent", seed=3)
+    p = E.default_params(box_len=s.spec.box_len, cutoff=s.spec.cutoff, dt=s.spec.dt, semantics=E.SEMANTICS_PHYSICS,
+                         skin=0.1, switch_on=1.0, nlist_period=0)
+    failed = []
+
+    def run(bins):
+        with E.Engine(s, p) as eng:
+            for _ in range(3000):
+                try:
+                    eng.rdf(bins, 1.0)
+                except E.LimaError as e:
+                    failed.append((bins, str(e)))
+                    return
+
+    threads = [threading.Thread(target=run, args=(b,)) for b in (128, 77) * 4]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed
