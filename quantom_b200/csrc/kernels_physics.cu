@@ -27,6 +27,8 @@
 // arrays) and k_build_list — one warp per one or four particles over the
 // columns of their 5x5x5 cell neighbourhood that their bounding box can
 // reach, which also copies the permuted arrays back.
+#include <type_traits>
+
 #include "cellrange.cuh"
 #include "physdev.cuh"
 #include "physkern.cuh"
@@ -1346,21 +1348,21 @@ void step_variant_lanes(const PhysDev& d, int cur, int slot, cudaGraphExec_t tai
 
 template <bool MIXED, bool ENERGY, bool INTEGRATE, bool TAIL, typename ID>
 void step_variant_id(const PhysDev& d, int cur, int slot, cudaGraphExec_t tail, cudaStream_t s) {
-    switch (step_lanes(d, ENERGY)) {
-#if !LIMA_STAGED_LIST
-        case 32: step_variant_lanes<32, MIXED, ENERGY, INTEGRATE, TAIL, ID>(d, cur, slot, tail, s); break;
-        case 16: step_variant_lanes<16, MIXED, ENERGY, INTEGRATE, TAIL, ID>(d, cur, slot, tail, s); break;
-#endif
-        default: step_variant_lanes<8, MIXED, ENERGY, INTEGRATE, TAIL, ID>(d, cur, slot, tail, s); break;
+    // more than 8 lanes: boxes whose ids are 16-bit; 16 lanes: without energies (step_lanes)
+    if constexpr (sizeof(ID) == 2) {
+        const int lanes = step_lanes(d, ENERGY);
+        if (lanes == 32) return step_variant_lanes<32, MIXED, ENERGY, INTEGRATE, TAIL, ID>(d, cur, slot, tail, s);
+        if constexpr (!ENERGY)
+            if (lanes == 16) return step_variant_lanes<16, MIXED, ENERGY, INTEGRATE, TAIL, ID>(d, cur, slot, tail, s);
     }
+    step_variant_lanes<8, MIXED, ENERGY, INTEGRATE, TAIL, ID>(d, cur, slot, tail, s);
 }
 
 template <bool MIXED, bool ENERGY, bool INTEGRATE, bool TAIL>
 void step_variant(const PhysDev& d, int cur, int slot, cudaGraphExec_t tail, cudaStream_t s) {
-    if (d.nl16)
-        step_variant_id<MIXED, ENERGY, INTEGRATE, TAIL, uint16_t>(d, cur, slot, tail, s);
-    else
-        step_variant_id<MIXED, ENERGY, INTEGRATE, TAIL, uint32_t>(d, cur, slot, tail, s);
+    if constexpr (!kStagedList)   // (the staged library's ids are 32-bit)
+        if (d.nl16) return step_variant_id<MIXED, ENERGY, INTEGRATE, TAIL, uint16_t>(d, cur, slot, tail, s);
+    step_variant_id<MIXED, ENERGY, INTEGRATE, TAIL, uint32_t>(d, cur, slot, tail, s);
 }
 
 template <bool MIXED, bool ENERGY, bool INTEGRATE>
@@ -1400,7 +1402,7 @@ void launch_set_xref(const PhysDev& d, const float4* pos, cudaStream_t s) {
     k_set_xref<<<(d.n + kTB - 1) / kTB, kTB, 0, s>>>(d, pos);
 }
 
-bool list_ids_16bit(int n_pad) { return !kStagedList && n_pad <= 65536; }
+bool list_ids_16bit(int n_pad) { return !kStagedList && n_pad <= kIds16Slots; }
 
 namespace {
 template <typename ID, int P>
@@ -1417,14 +1419,12 @@ void build_list(const PhysDev& d, const float4* pos, const uint32_t* orig, const
 
 void launch_build_list(const PhysDev& d, const float4* pos, const uint32_t* orig, const uint32_t* items, int copy_cur,
                        bool mixed, cudaStream_t s) {
-    // (measured at kBuildOneBelow)
-    if (d.n < kBuildOneBelow) {
-        if (d.nl16) build_list<uint16_t, 1>(d, pos, orig, items, copy_cur, mixed, s);
-        else build_list<uint32_t, 1>(d, pos, orig, items, copy_cur, mixed, s);
-    } else {
-        if (d.nl16) build_list<uint16_t, 4>(d, pos, orig, items, copy_cur, mixed, s);
-        else build_list<uint32_t, 4>(d, pos, orig, items, copy_cur, mixed, s);
-    }
+    // (measured at kBuildOneBelow; boxes below it have this library's narrowest ids)
+    using Narrow = typename std::conditional<kStagedList, uint32_t, uint16_t>::type;
+    if (d.n < kBuildOneBelow) return build_list<Narrow, 1>(d, pos, orig, items, copy_cur, mixed, s);
+    if constexpr (!kStagedList)
+        if (d.nl16) return build_list<uint16_t, 4>(d, pos, orig, items, copy_cur, mixed, s);
+    build_list<uint32_t, 4>(d, pos, orig, items, copy_cur, mixed, s);
 }
 
 namespace {

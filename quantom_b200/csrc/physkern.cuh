@@ -68,15 +68,15 @@ __host__ __device__ inline int nl_round_cap(int want) { return (want + kListChun
 __device__ __forceinline__ uint32_t nl_load(const PhysDev& d, size_t idx) {
     return d.nl16 ? (uint32_t)reinterpret_cast<const uint16_t*>(d.nl)[idx] : d.nl[idx];
 }
-__device__ __forceinline__ void nl_store(const PhysDev& d, size_t idx, uint32_t j) {
-    if (d.nl16)
-        reinterpret_cast<uint16_t*>(d.nl)[idx] = (uint16_t)j;
-    else
-        d.nl[idx] = j;
-}
 // whether the step kernels of this library take 16-bit list ids for n_pad
 // slots: whenever they fit, except in the staged variant (32-bit rows)
+constexpr int kIds16Slots = 65536;
 bool list_ids_16bit(int n_pad);
+// the step kernels of more than 8 lanes and the list build of one particle a
+// warp exist for 16-bit ids alone (in the staged library the build's are 32-bit)
+static_assert(kStep32Below <= kStep16Below && kStep16Below < kIds16Slots && kStepEnergy32Below < kIds16Slots &&
+                  kBuildOneBelow < kIds16Slots,
+              "small-box kernels take 16-bit ids");
 // bytes of one list entry
 __host__ __device__ inline size_t nl_entry_bytes(const PhysDev& d) { return d.nl16 ? 2 : 4; }
 
