@@ -101,3 +101,21 @@ def test_threads_with_different_bins():
     for t in threads:
         t.join()
     assert not failed
+
+
+@pytest.mark.parametrize("bins", [1, 50])
+def test_occupancies_do_not_depend_on_the_particle_order(bins):
+    """Occupancies are exact sums of the pairs' weights (integers in units of
+    2^-32; with 4,096 particles every partial sum is exact in FP64 too): the same
+    box with its waters in another order gives the same bits.  One bin takes the
+    32-bit columns past 2^32 many times."""
+    from dataclasses import replace
+    s = S.make_system("lj_solvent_4096", seed=3)
+    p = E.default_params(box_len=s.spec.box_len, cutoff=s.spec.cutoff, dt=s.spec.dt, semantics=E.SEMANTICS_PHYSICS,
+                         skin=0.1, switch_on=1.0, nlist_period=0)
+    order = np.random.default_rng(8).permutation(s.n_solvents)
+    h = []
+    for t in (s, replace(s, solvents=s.solvents[order].copy())):
+        with E.Engine(t, p) as eng:
+            h.append(eng.rdf(bins, 1.2 * bins / (bins + 1) * 0.999))
+    assert np.array_equal(h[0], h[1])
