@@ -33,13 +33,6 @@ constexpr int kListEpoch = 10;
 
 __device__ __forceinline__ float mimg_a(float d, float L, float invL) { return d - L * rintf(d * invL); }
 
-// 1 / x to about half an ulp: the special-function unit's reciprocal and one
-// Newton step (x positive, far from the denormal and overflow ranges)
-__device__ __forceinline__ float rcp_newton(float x) {
-    const float r = rcp_approx(x);
-    return fmaf(r, fmaf(-x, r, 1.f), r);
-}
-
 // f(slot j, position) for one lane's entries of particle i's list, of the LANES
 // lanes that share it: lane 8 h + g takes column g of the chunks h, h + LANES /
 // 8, ... (nl_word), four entries per vector load and four gathers in flight.
@@ -496,7 +489,7 @@ __global__ void __launch_bounds__(kAdjPairTB) k_adj_pair(PhysDev d, const float4
                     bspline3(r, a.inv_dr, k0, wt, dw);
                     k0 = min(k0, kmax);   // past the support: zeros
                     const float* c = s_c + k0 + 1;
-                    const float G = (c[0] * dw[0] + c[1] * dw[1] + c[2] * dw[2]) * rcp_newton(r);
+                    const float G = quot_newton(c[0] * dw[0] + c[1] * dw[1] + c[2] * dw[2], r);
                     rx += G * dx;
                     ry += G * dy;
                     rz += G * dz;
