@@ -413,7 +413,8 @@ __device__ __forceinline__ void scan_stream(const PhysDev& d, const float4* __re
             r2 = qe == p ? nan : r2;   // not itself
             append_hits<ID>(r2, rl2, __float_as_uint(e.w), lt, end[p], at[p]);
         }
-        if (cap < (uint32_t)d.nl_cap) {   // rows shorter than the list's: to the list before one can run over
+        // rows shorter than the list's and the exclusions still in them: to the list before one can run over
+        if (cap < (uint32_t)(d.nl_cap + d.excl_max)) {
             uint32_t room = end[0] - at[0];
 #pragma unroll
             for (int p = 1; p < P; p++) room = min(room, end[p] - at[p]);
@@ -570,17 +571,18 @@ __global__ void __launch_bounds__(kBuildWarps * 32, P == 1 ? 8 : 0) k_build_list
                                                  px, py, pz, row, (uint32_t)cap, cnt, lane);
         }
     }
-    uint32_t found[P];   // before the exclusions: what a row may have run over the list's capacity by
+    uint32_t lost[P];   // hits past the end of a row: more than the list and the exclusions take
 #pragma unroll
-    for (int p = 0; p < P; p++) found[p] = done[p] + cnt[p];
+    for (int p = 0; p < P; p++) lost[p] = cnt[p] - min(cnt[p], (uint32_t)cap);
     flush_rows<ID, P>(d, orig, rows, cap, i, base, true, cnt, done, lane);
 #pragma unroll
     for (int p = 0; p < P; p++)
         if (lane == p && have) {
-            d.nl_cnt[i] = min(done[p] + cnt[p], (uint32_t)d.nl_cap);
-            if (found[p] > (uint32_t)d.nl_cap) {
+            const uint32_t found = done[p] + cnt[p] + lost[p];
+            d.nl_cnt[i] = min(found, (uint32_t)d.nl_cap);
+            if (found > (uint32_t)d.nl_cap) {
                 atomicOr(d.err, ERR_BIT_PHYS_LIST_OVERFLOW);
-                atomicMax(d.nl_need, (int)found[p]);
+                atomicMax(d.nl_need, (int)found);
             }
         }
 }
@@ -1409,7 +1411,8 @@ template <typename ID, int P>
 void build_list(const PhysDev& d, const float4* pos, const uint32_t* orig, const uint32_t* items, int copy_cur,
                 bool mixed, cudaStream_t s) {
     const int warps = (d.n + P - 1) / P;
-    const int cap = std::min(d.nl_cap, kBuildRow);
+    // room for the exclusions too: a row overflows by what is left without them
+    const int cap = std::min(nl_round_cap(d.nl_cap + d.excl_max), kBuildRow);
     const size_t smem = kBuildWarps * build_warp_smem(P, cap, sizeof(ID));
     allow_smem(k_build_list<ID, P>, smem, 0, kBuildWarps * build_warp_smem(P, kBuildRow, sizeof(ID)));
     k_build_list<ID, P><<<(warps + kBuildWarps - 1) / kBuildWarps, kBuildWarps * 32, smem, s>>>(

@@ -104,7 +104,7 @@ struct PhysDev {
     unsigned long long* rebuild_count;   // rebuilds launched from the device
     cudaGraphExec_t rebuild_exec[2];     // device-launchable rebuild of pos[parity] (null: host decides)
     // exclusions (CSR over orig ids)
-    uint32_t* excl_off; uint32_t* excl_ids;
+    uint32_t* excl_off; uint32_t* excl_ids; int excl_max;   // CSR by orig id, its longest row
     // bonded terms (orig ids); a term slot numbers (term, role): bond b role r
     // -> 2b + r, angle a -> 2 n_bonds + 3a + r, dihedral q -> 2 n_bonds +
     // 3 n_angles + 4q + r

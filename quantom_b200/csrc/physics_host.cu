@@ -210,6 +210,7 @@ int phys_setup(const PhysHost& h, PhysDev& d, cudaStream_t s, std::vector<void*>
     for (int i = 0; i < d.n; i++) {
         eoff[i + 1] = eoff[i] + (i < d.n_cp ? (uint32_t)excl[i].size() : 0u);
         if (i < d.n_cp) eids.insert(eids.end(), excl[i].begin(), excl[i].end());
+        d.excl_max = std::max(d.excl_max, (int)(eoff[i + 1] - eoff[i]));
     }
     // bonded terms with orig ids (compounds, then bridges)
     std::vector<int4> bidx, aidx, didx;

@@ -126,3 +126,46 @@ def test_rebuild_with_particles_thrown_out_of_the_box(apart, axis):
         eng.set_state(s.states, None, s.solvents)
         goff, gids = eng.nlist(E.NL_PAIR)
         assert np.array_equal(goff, off) and np.array_equal(gids, ids)
+
+
+@pytest.mark.parametrize("box,waters", [(10.0, 1000), (20.0, 17000)])   # one and four particles a warp
+@pytest.mark.parametrize("beyond", [0, 1])
+def test_capacity_counts_rows_without_their_exclusions(box, waters, beyond):
+    """A row that fits the list once its bonded exclusions are out of it is
+    accepted; one entry more is a capacity status.  A straight chain in the
+    middle, its middle particle's neighbours in two clusters of waters that do
+    not see each other, the other waters on a sparse lattice."""
+    length, mid = 24, 12
+    spec = S.SystemSpec("box", box, waters, cutoff=0.9, chains=S.ChainSpec(1, length), mc_sweeps=0)
+    s = S.make_system(spec, seed=14)
+    skin = 0.1
+    n = length + waters
+    # the list's capacity (a third more than an even density fills, and 96, in chunks of 32)
+    cap = (int(1.6 * (4 / 3 * np.pi * 1.0 ** 3 * n / box ** 3) + 96) + 31) // 32 * 32
+    excl = int(s.compounds[0]["lj_ignore_list"][mid]["n_ignores"])
+    near = 8                                         # chain particles within 1 nm of the middle one
+    assert 1 < excl < near
+    in_reach = cap + beyond - (near - excl)          # waters in its list
+    c = box / 2
+    st, sol = s.states.copy(), s.solvents.copy()
+    st["positions"][0, :length] = c
+    st["positions"][0, :length, 1] += 0.21 * (np.arange(length) - mid)
+    rng = np.random.default_rng(2)
+    x = rng.uniform(-0.01, 0.01, (in_reach, 3)) + c
+    x[:, 0] += np.where(np.arange(in_reach) % 2, 0.93, -0.93)
+    g = (np.stack(np.meshgrid(*[np.arange(int(box / 0.72))] * 3), -1).reshape(-1, 3) + 0.5) * 0.72
+    g = g[np.linalg.norm(g - c, axis=1) > 4.0]
+    sol["pos"] = np.concatenate([x, g[: waters - in_reach]])
+    p = E.default_params(box_len=box, cutoff=0.9, dt=spec.dt, semantics=E.SEMANTICS_PHYSICS, skin=skin, switch_on=0.8,
+                         nlist_period=0)
+    with E.Engine(s, p) as eng:
+        if beyond:
+            with pytest.raises(E.LimaError) as ei:
+                eng.set_state(st, None, sol)
+            assert ei.value.status == E.ERR_CAPACITY
+        else:
+            eng.set_state(st, None, sol)
+            off, ids = eng.nlist(E.NL_PAIR)
+            assert off[mid + 1] - off[mid] == cap
+            mine = ids[off[mid]:off[mid + 1]]
+            assert (mine < length).sum() == near - excl and (mine >= length).sum() == in_reach
