@@ -901,7 +901,8 @@ lima_status lima_get_positions(lima_ctx* c, float* cxyz, float* sxyz) {
         const int nc = static_cast<int>(c->comps.size()), ns = static_cast<int>(c->sols.size());
         const size_t ncp = static_cast<size_t>(nc) * lima::kMaxCP;
         if (c->p.semantics == LIMA_SEMANTICS_PHYSICS) {
-            // one kernel writes both flat arrays on the device, one copy each into the caller's, one wait
+            // one kernel writes both flat arrays on the device; the one wait raises what the steps
+            // flagged before anything reaches the caller's arrays
             if ((!cxyz || nc == 0) && (!sxyz || ns == 0)) {
                 sync_checked(c);
                 return;
@@ -910,11 +911,12 @@ lima_status lima_get_positions(lima_ctx* c, float* cxyz, float* sxyz) {
             lima_float3* dc = cxyz && nc > 0 ? g.prev : nullptr;
             lima_float3* ds = sxyz && ns > 0 ? reinterpret_cast<lima_float3*>(g.sols) : nullptr;
             lima::launch_read_positions(c->phys, c->cur, dc, ds, c->stream);
+            sync_checked(c);
             if (dc)
                 cuda_ok(cudaMemcpyAsync(cxyz, dc, sizeof(lima_float3) * ncp, cudaMemcpyDeviceToHost, c->stream), "D2H");
             if (ds)
                 cuda_ok(cudaMemcpyAsync(sxyz, ds, sizeof(lima_float3) * ns, cudaMemcpyDeviceToHost, c->stream), "D2H");
-            sync_checked(c);
+            cuda_ok(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
             return;
         }
         sync_checked(c);

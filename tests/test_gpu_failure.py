@@ -30,3 +30,23 @@ def test_overflowing_forces_are_a_numeric_status(gpu):
         # the context still answers: the flags were cleared when reported
         eng.synchronize()
         assert len(eng.solvents()) == s.n_solvents
+
+
+def test_positions_of_a_failed_step_leave_the_arrays_alone(gpu):
+    """lima_get_positions raises what the steps before it flagged and writes
+    neither of the caller's arrays; asked again it answers."""
+    E = gpu
+    s = S.make_system("tiny_chains", seed=3)
+    p = E.default_params(box_len=s.spec.box_len, cutoff=s.spec.cutoff, dt=s.spec.dt,
+                         semantics=E.SEMANTICS_PHYSICS, skin=0.1, switch_on=1.0, nlist_period=10)
+    bad = s.solvents.copy()
+    bad["pos"][1, 0] = np.nan
+    c = np.full((s.n_compounds, 64, 3), -7.0, np.float32)
+    x = np.full((s.n_solvents, 3), -7.0, np.float32)
+    with E.Engine(s, p) as eng:
+        eng.set_state(s.states, None, bad)
+        eng.step(1)
+        assert eng.lib.lima_get_positions(eng.h, c.ctypes.data, x.ctypes.data) == E.ERR_NUMERIC
+        assert (c == -7.0).all() and (x == -7.0).all()
+        assert eng.lib.lima_get_positions(eng.h, c.ctypes.data, x.ctypes.data) == E.OK
+        assert (c != -7.0).all() and (x != -7.0).all()
