@@ -1025,8 +1025,7 @@ lima_status lima_compute_energies(lima_ctx* c) {
             c->launches += lima::rebuild_kernels(c->phys);
             c->host_rebuilds++;
         }
-        lima::phys_energy_now(c->phys, c->cur, c->stream);
-        c->launches += 2;
+        c->launches += lima::phys_energy_now(c->phys, c->cur, c->stream);
         sync_checked(c);
     });
 }

@@ -187,7 +187,7 @@ inline int rebuild_kernels(const PhysDev& d) { return d.n < kPermuteAloneFrom ? 
 // kernel, after it, after the step kernel.  Returns kernels launched.
 int phys_step_kernels(const PhysDev& d, int cur, cudaStream_t s, bool energy = false, cudaEvent_t* ev = nullptr,
                       bool tail = false);
-void phys_energy_now(PhysDev& d, int cur, cudaStream_t s);
+int phys_energy_now(PhysDev& d, int cur, cudaStream_t s);   // returns the kernels launched
 // Host copy of the state in orig order (position and previous position, in
 // double), kept while the state it was read from is unchanged: `key` names
 // that state (the caller changes it whenever the state may have changed).

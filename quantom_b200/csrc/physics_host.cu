@@ -628,9 +628,10 @@ int phys_step_kernels(const PhysDev& d, int cur, cudaStream_t s, bool energy, cu
     return 1 + bonded;
 }
 
-void phys_energy_now(PhysDev& d, int cur, cudaStream_t s) {
-    launch_bonded(d, cur, true, s);
+int phys_energy_now(PhysDev& d, int cur, cudaStream_t s) {
+    const int bonded = launch_bonded(d, cur, true, s);
     launch_step(d, cur, d.precision == LIMA_PRECISION_MIXED, true, false, kSlotEval, nullptr, s);
+    return 1 + bonded;
 }
 
 namespace {

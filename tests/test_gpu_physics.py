@@ -262,3 +262,14 @@ def test_verlet_list_matches_brute_force(gpu, name):
         assert must <= got, (i, sorted(must - got)[:5])
         assert got <= may, (i, sorted(got - may)[:5])
         assert not any((i, j) in excl for j in got)
+
+
+@pytest.mark.parametrize("name,kernels", [("tiny_chains", 2), ("tiny_solvent", 1)])
+def test_energy_evaluation_counts_its_kernels(gpu, name, kernels):
+    """compute_energies launches the bonded kernel only where there are bonded terms."""
+    E = gpu
+    s = S.make_system(name, seed=3)
+    with E.Engine(s, _params(E, s)) as eng:
+        before = eng.kernel_launches()
+        eng.compute_energies()
+        assert eng.kernel_launches() - before == kernels
