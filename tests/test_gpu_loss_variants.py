@@ -119,3 +119,29 @@ def test_occupancies_do_not_depend_on_the_particle_order(bins):
         with E.Engine(t, p) as eng:
             h.append(eng.rdf(bins, 1.2 * bins / (bins + 1) * 0.999))
     assert np.array_equal(h[0], h[1])
+
+
+@pytest.mark.parametrize("box,waters,entries", [(4.0, 1901, 2),      # 16 lanes
+                                                (6.0, 6150, 2),      # 8 lanes
+                                                (13.0, 66003, 1)])   # 32-bit ids
+def test_gradient_of_a_chain_type(box, waters, entries):
+    """The derivatives that land on another type than the waters' (in the lane's
+    own columns): sigma and epsilon of the last chain type."""
+    from oracle import pyoracle as po
+    s, p = _box(box, waters, 2, 24)
+    bins, steps = 20, 2
+    r_max = 1.2 * bins / (bins + 1) * 0.999
+    ps = po.PhysSystem(s, rc=1.2, r_on=1.0)
+    target = 0.97 * ps.rdf(bins, r_max)
+    with E.Engine(s, p) as eng:
+        _, g = eng.grad(steps, 2, bins, r_max, 1.0, 100.0, target)
+        n_types = eng.param_layout()["n_types"]
+    th = ps.params()
+    value = lambda t: ps.with_params(t).loss(s.spec.dt, steps, bins, r_max, 1.0, 100.0, target)[0]  # noqa: E731
+    kind = int(s.compounds[0]["atom_types"][: s.compounds[0]["n_particles"]].max())
+    assert kind > 0
+    for k in (kind, n_types + kind)[:entries]:
+        e = np.zeros(len(th))
+        e[k] = 1e-4 * abs(th[k])
+        fd = (value(th + e) - value(th - e)) / (2 * e[k])
+        assert abs(g[k] - fd) < 1e-3 * abs(fd), (k, g[k], fd)
