@@ -414,7 +414,7 @@ __device__ __forceinline__ void scan_stream(const PhysDev& d, const float4* __re
             append_hits<ID>(r2, rl2, __float_as_uint(e.w), lt, end[p], at[p]);
         }
         // rows shorter than the list's and the exclusions still in them: to the list before one can run over
-        if (cap < (uint32_t)(d.nl_cap + d.excl_max)) {
+        if (cap < (uint32_t)d.nl_room) {
             uint32_t room = end[0] - at[0];
 #pragma unroll
             for (int p = 1; p < P; p++) room = min(room, end[p] - at[p]);
@@ -1412,7 +1412,7 @@ void build_list(const PhysDev& d, const float4* pos, const uint32_t* orig, const
                 bool mixed, cudaStream_t s) {
     const int warps = (d.n + P - 1) / P;
     // room for the exclusions too: a row overflows by what is left without them
-    const int cap = std::min(nl_round_cap(d.nl_cap + d.excl_max), kBuildRow);
+    const int cap = std::min(nl_round_cap(d.nl_room), kBuildRow);
     const size_t smem = kBuildWarps * build_warp_smem(P, cap, sizeof(ID));
     allow_smem(k_build_list<ID, P>, smem, 0, kBuildWarps * build_warp_smem(P, kBuildRow, sizeof(ID)));
     k_build_list<ID, P><<<(warps + kBuildWarps - 1) / kBuildWarps, kBuildWarps * 32, smem, s>>>(

@@ -92,6 +92,7 @@ struct PhysDev {
     float4* pos_tmp[2]; float4* vel_tmp; float4* posc_tmp; float4* velc_tmp; float4* force_tmp; uint32_t* orig_tmp;
     // Verlet list (tile-local indices)
     uint32_t* nl; uint32_t* nl_cnt; int nl_cap;
+    int nl_room;                // nl_cap + excl_max: hits of a particle that can fit the list once its exclusions are out
     int nl16;                   // 1: nl holds uint16 slot ids (half the bytes per step), 0: uint32
     int* nl_need;               // largest row length a build found beyond nl_cap (0: none)
     // dynamic lists (nlist_period <= 0): the step kernel's last block sees

@@ -300,6 +300,7 @@ int phys_setup(const PhysHost& h, PhysDev& d, cudaStream_t s, std::vector<void*>
     const double expect = 4.0 / 3.0 * M_PI * (double)d.rlist * d.rlist * d.rlist * rho;
     d.nl_cap = std::min(nl_round_cap(d.n), nl_round_cap((int)(1.6 * expect + 96)));
     d.nl_cap = std::max(d.nl_cap, kListChunk);
+    d.nl_room = d.nl_cap + d.excl_max;
     d.nl16 = list_ids_16bit(d.n_pad) ? 1 : 0;
 
     // every fixed-size buffer in one allocation; the list separately (it may grow)
@@ -518,6 +519,7 @@ bool phys_fit_list(PhysDev& d, cudaStream_t s, std::vector<void*>& allocs) {
         }
     d.nl = nl;
     d.nl_cap = cap;
+    d.nl_room = cap + d.excl_max;
     const int zero = 0;
     const int keep = err & ~ERR_BIT_PHYS_LIST_OVERFLOW;
     cudaMemcpyAsync(d.err, &keep, sizeof(int), cudaMemcpyHostToDevice, s);
