@@ -398,9 +398,9 @@ __global__ void k_adj_prep(PhysDev d, AdjArgs a, float4* __restrict__ lam_v, flo
     wv[i] = make_float4(mx * im, my * im, mz * im, 0.f);
 }
 
-// kGroup lanes per particle (pair_lanes).  Every entry is evaluated (beyond r_c the switch and
-// its derivatives are zero, beyond the last bin the staged occupancy error is),
-// so a warp's lanes stay together.  The quotients of the per-type chain rule
+// LANES lanes (8 or 16, pair_lanes) per particle.  Every entry is evaluated
+// (beyond r_c the switch and its derivatives are zero, beyond the last bin the
+// staged occupancy error is), so a warp's lanes stay together.  The quotients of the per-type chain rule
 // (sigma_ij = (s_a + s_b) / 2, eps_ij = sqrt(e_a e_b)) are a table per type
 // pair.  The derivatives that land on the neighbour's type go to a column of
 // the lane's own in shared memory ([2 types][32] per warp: no conflicts, no
@@ -418,9 +418,9 @@ __global__ void __launch_bounds__(kAdjPairTB) k_adj_pair(PhysDev d, const float4
                                                          const double* __restrict__ hist_n,
                                                          const double* __restrict__ target) {
     extern __shared__ float4 s_dyn[];
-    // per type pair: (sigma^2, 4 eps, 1 / sigma, 0) and d eps_ij / d eps of i's and j's type
     __shared__ float s_c[LIMA_LOSS_MAX_BINS + 8];   // occupancy error of bin b at b + 1, zero outside
     const int nt = a.n_types;
+    // per type pair: (sigma^2, 4 eps, 1 / sigma, 0) and d eps_ij / d eps of i's and j's type
     float4* s_tab = s_dyn;
     float2* s_de = reinterpret_cast<float2*>(s_dyn + nt * nt);
     float* s_g = reinterpret_cast<float*>(s_de + nt * nt + (nt * nt & 1));   // [warps][2 nt][32]
@@ -781,7 +781,9 @@ namespace {
 // 40 steps of 5,040 particles 5.54, 5.25, 5.82; 200 steps of 8,192 particles
 // 26.3, 27.6, 30.8 (with the loss kernel on as many lanes).  The loss kernel
 // keeps 8: more lanes are more columns of occupancies to clear and sum (200
-// steps of 8,192 particles: 11.5 ms with 8, 14.1 with 16).
+// steps of 8,192 particles: 11.5 ms with 8, 14.1 with 16).  The line lies between
+// 5,040 and 8,192; no size between them was measured, nor another cutoff, which
+// changes the list a lane walks.
 int pair_lanes(int n) { return n < 6144 ? 16 : kGroup; }
 
 struct Runner {

@@ -226,9 +226,9 @@ __global__ void k_set_xref(PhysDev d, const float4* __restrict__ pos) {
 // particle walking the candidates took ~50 instructions per 32 tests for hit
 // masks, ranks and branches), loops run on values the compiler knows to be
 // uniform, exclusions cost only the rows that have any, and small boxes put
-// one particle on a warp (kBuildOneBelow).  A host-issued rebuild, sort and
-// launches included, on one B200 (before -> now): 4,096 particles 110 -> 47
-// us, 8,192 120 -> 61, 32,024 153 -> 110, 258,192 683 -> 557.
+// one particle on a warp (kBuildOneBelow).  A host-issued rebuild, sort,
+// launches and synchronisation included, on one B200 (before -> now): 4,096
+// particles 118 -> 45 us, 8,192 123 -> 58, 32,024 158 -> 112, 258,192 687 -> 575.
 // pos/orig: positions and orig ids by slot.  items (nullable): the cell order
 // as a list of slots when the particles were not moved into it (in-place
 // rebuild).  copy_cur >= 0: the particles were permuted into the tmp arrays
@@ -1100,7 +1100,7 @@ __device__ __forceinline__ void step_body(const PhysDev& d, int cur, int slot, c
     float e_i = 0.f, w_i = 0.f;
     const int cnt = active ? (int)d.nl_cnt[i] : 0;
     // the axes that take the minimum image: those on which some particle of the
-    // warp lies within r_c of a face (one axis alone, or all three)
+    // warp lies within r_c of a face (one axis alone, x and y, or all three)
     const unsigned wm = __reduce_or_sync(0xffffffffu, active ? face_axes(d, pi) : 0u);
 #if LIMA_STAGED_LIST
     const int rows = cnt > g ? (cnt - g + kGroup - 1) / kGroup : 0;   // this lane's entries: g, g + 8, ... below cnt

@@ -177,7 +177,8 @@ void phys_free_rebuild(PhysDev& d);
 // From this box size on the rebuild moves the per-slot arrays in a kernel of its
 // own, a thread per slot; below, the warp that orders a cell moves its slots
 // too (about a third of its lanes have one: 32,024 particles a host-issued
-// rebuild 106 -> 103 us with the launch it saves, 258,192 565 -> 592).
+// rebuild 106 -> 103 us with the launch it saves, 258,192 565 -> 592; no size
+// between them was measured).
 constexpr int kPermuteAloneFrom = 131072;
 // k_sort_count, k_sort_fill, k_sort_order, (k_permute), k_build_list
 inline int rebuild_kernels(const PhysDev& d) { return d.n < kPermuteAloneFrom ? 4 : 5; }

@@ -14,7 +14,8 @@ constexpr int kBuildWarps = 4;   // warps per block of the list build
 // shorter streams) and four from it on (fewer tests and one stream's fetches
 // for four).  A host-issued rebuild with 1 / 4 particles a warp: 4,096
 // particles 61 / 72 us, 8,192 76 / 78, 32,024 136 / 124, 258,192 748 / 571
-// (14 us of each the call's synchronisation).
+// (14 us of each the call's synchronisation).  No size between 8,192, where the two
+// are level, and 32,024 was measured.
 constexpr int kBuildOneBelow = 16384;
 constexpr int kMaxTypes = 32;    // LIMA_MAX_ATOM_TYPES
 constexpr int kScanThreads = 1024;
@@ -39,7 +40,8 @@ inline void allow_smem(K kernel, size_t dynamic, size_t fixed, size_t most) {
 // 16.3 / 15.0 / 14.2 us, 1,948 17.5 / 16.3 / 15.8, 4,096 18.3 / 16.6 / 18.6,
 // 8,192 20.1 / 21.4 / 23.1.  With energies (more sums to reduce, and the frame
 // behind it) 200 steps: 880 4.60 / 4.52 / 3.97 ms, 1,948 4.72 / 5.11 / 5.09,
-// 3,893 4.99 / 5.11 / 5.77.
+// 3,893 4.99 / 5.11 / 5.77.  The lines lie between these sizes (at a 1.2 nm cutoff,
+// ~295 entries a list); none between them was measured, nor another cutoff.
 constexpr int kStep32Below = 2048, kStep16Below = 6144, kStepEnergy32Below = 1024;
 // the step kernel reads its list rows from shared memory, staged by bulk
 // copies in groups of kStageRows rows (false: per-lane loads from the list).
